@@ -263,12 +263,27 @@ static const std::vector<const void *> *jit_backward(const mqb_program &p, Sched
     return &v;
 }
 
-static std::unique_ptr<SchedDev> make_sched(const mqb_program &p, int K, bool fuse, int reg_bits) {
+// Matrix-table entries a pass may hold so that the tile ring of its generated kernel (two groups, each with
+// its own table and gradient slots) keeps three buffers in 227 KB, or two where three leave less than 8 KB
+// for a table.  n_hams = 0: a forward schedule.
+static PassLimits pass_limits(const mqb_program &p, int K, int reg_bits, int n_hams) {
+    const int64_t buf = (int64_t(1) << K) * int64_t(p.elem()) * (1 + n_hams);
+    const int64_t slots = int64_t(1 << std::max(0, K - reg_bits - 5)) * kMaxPassSlots * n_hams * int64_t(sizeof(double));
+    auto table = [&](int buffers) { return ((int64_t(227) << 10) - 256 - buffers * buf) / 2 - slots; };
+    const int64_t bytes = table(3) >= 8192 ? table(3) : table(2);
+    PassLimits lim;
+    lim.max_entries = int(std::max<int64_t>(bytes, 4096) / int64_t(p.elem()));
+    lim.derivatives = n_hams > 0;
+    return lim;
+}
+
+static std::unique_ptr<SchedDev> make_sched(const mqb_program &p, int K, bool fuse, int reg_bits, int n_hams) {
     auto sd = std::make_unique<SchedDev>();
     // the register kernels need 2^5..2^8 threads of 2^reg_bits amplitudes: smaller registers use
     // the per-gate kernels
     if (K < reg_bits + 5) fuse = false;
-    sd->s = build_schedule(p.n, K, contiguity_bits(p.precision), p.ops, fuse, &p.no_fuse);
+    sd->s = build_schedule(p.n, K, contiguity_bits(p.precision), p.ops, fuse, &p.no_fuse,
+                           pass_limits(p, K, reg_bits, n_hams));
     build_stages(sd->s, p.ops, reg_bits, p.precision, false);
     build_stages(sd->s, p.ops, fwd_reg_bits(p.precision), p.precision, true);
     sd->s.d_pass_ops = upload(sd->s.pass_ops);
@@ -295,7 +310,7 @@ static SchedDev &grad_schedule(mqb_program &p, int n_hams) {
     auto it = p.grad_sched.find(key);
     if (it != p.grad_sched.end()) return *it->second;
     const int rb = bwd_reg_bits(p.precision, n_hams);
-    auto sd = make_sched(p, fused ? tile_bits_for(p, rb) : p.n, fused, rb);
+    auto sd = make_sched(p, fused ? tile_bits_for(p, rb) : p.n, fused, rb, n_hams);
     SchedDev &ref = *sd;
     p.grad_sched[key] = std::move(sd);
     return ref;
@@ -958,7 +973,7 @@ int mqb_program_create(int n_qubits, int precision, const mqb_gate_desc *gates, 
         p->d_csr_slot = upload(slot);
         p->d_csr_coeff = upload(coeff);
         const int rb = fwd_reg_bits(precision);
-        p->apply_sched = make_sched(*p, tile_bits_for(*p, rb), p->fuse != 0, rb);
+        p->apply_sched = make_sched(*p, tile_bits_for(*p, rb), p->fuse != 0, rb, 0);
         *out = p.release();
     });
 }

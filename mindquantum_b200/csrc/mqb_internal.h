@@ -192,10 +192,16 @@ class JitBlock {
     bool prev_;
 };
 
+// What one fused pass may hold besides kMaxPassOps and kMaxPassSlots.
+struct PassLimits {
+    int max_entries = 1 << 30;   // complex entries of the pass's shared-memory matrix table
+    bool derivatives = true;     // whether the table holds the gates' derivative matrices too
+};
+
 // Builders (scheduler.cpp)
 // no_fuse (optional, one entry per op): ops that must run in a pass of their own.
 Schedule build_schedule(int n, int K, int c, const std::vector<DevOp> &ops, bool fuse,
-                        const std::vector<char> *no_fuse = nullptr);
+                        const std::vector<char> *no_fuse = nullptr, const PassLimits &limits = PassLimits());
 // Split every fused pass of `s` into register stages with `reg_bits` register bits per thread:
 // the backward layout (Schedule::stages) or, with `forward`, the forward layout (f_stages).
 void build_stages(Schedule &s, const std::vector<DevOp> &ops, int reg_bits, int precision, bool forward = false);

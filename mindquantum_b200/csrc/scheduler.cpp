@@ -7,11 +7,13 @@
 // read + write of the state, every gate whose non-diagonal targets lie in Q.  Diagonal gates
 // and control qubits may sit anywhere: outside Q their bits are constant over a tile.
 //
-// The greedy scan keeps the circuit's order of non-commuting gates: a gate that cannot join
+// The greedy scan keeps the circuit's order of gates that share a qubit: a gate that cannot join
 // the current pass blocks all its qubits for the rest of the scan, so no later gate sharing a
-// qubit with it can overtake it.
+// qubit with it can overtake it.  The set Q of a pass (and the register bits of a stage) is the one
+// of several candidates that takes the most gates (choose_set).
 #include <algorithm>
 #include <cstdlib>
+#include <iterator>
 #include <stdexcept>
 
 #include "mqb_internal.h"
@@ -75,7 +77,140 @@ static uint64_t touched(const DevOp &op) {
 
 static bool fusable(const DevOp &op) { return (op.kind == KIND_DENSE || op.kind == KIND_DIAG) && op.m <= kMaxFusedM; }
 
-Schedule build_schedule(int n, int K, int c, const std::vector<DevOp> &ops, bool fuse, const std::vector<char> *no_fuse) {
+namespace {
+
+// One item of a greedy scan (a gate in build_schedule, a pass op in build_stages): the qubits (bits)
+// it touches, the ones that have to be in the chosen set, and what it adds to the limits.
+struct ScanItem {
+    uint64_t touch = 0, dense = 0;
+    int slots = 0, entries = 0;
+    bool fusable = true;
+};
+
+struct ScanLimits {
+    int K = 0;                       // qubits of the set
+    int max_items = 1 << 30, max_slots = 1 << 30, max_entries = 1 << 30;
+    uint64_t all = 0;
+};
+
+// The items of `left` (indices, in program order) that can run together when the set is Q, which
+// grows up to K qubits as the items ask for them when `grow`.  An item that cannot join blocks the
+// qubits it touches for the rest of the scan.  Returns how many join; `members` may be null.
+int scan_items(const std::vector<ScanItem> &items, const std::vector<int> &left, const ScanLimits &lim, uint64_t &Q,
+               bool grow, std::vector<int> *members) {
+    uint64_t blocked = 0;
+    int n_items = 0, n_slots = 0, n_entries = 0;
+    for (int i : left) {
+        const ScanItem &it = items[i];
+        if (n_items >= lim.max_items) break;
+        const uint64_t need = it.dense & ~Q;
+        if ((it.touch & blocked) || !it.fusable || (need && (!grow || popc(Q | need) > lim.K)) ||
+            n_slots + it.slots > lim.max_slots || n_entries + it.entries > lim.max_entries) {
+            blocked |= it.touch;
+            if ((blocked & lim.all) == lim.all) break;
+            continue;
+        }
+        Q |= need;
+        n_slots += it.slots;
+        n_entries += it.entries;
+        ++n_items;
+        if (members) members->push_back(i);
+    }
+    return n_items;
+}
+
+// The set of at most K qubits, Q0 among them, under which the most items of `left` run together, out
+// of: the qubits in the order the items ask for them; every window of consecutive qubits above
+// Q0 (`windows`); and Q0 grown by the qubit that lets most items join, one at a time.  In a layered circuit a
+// set taken in program order is used for about two layers: the gates of later layers wait for
+// neighbours outside it.  A window next to the qubits that earlier passes brought furthest lets a
+// wedge of many layers through (26 qubits x 12 layers of RY, RZ and a CNOT ladder, 12-qubit sets: 14
+// passes instead of 31).  Ties keep the program-order set.
+uint64_t choose_set(const std::vector<ScanItem> &items, const std::vector<int> &left, const ScanLimits &lim,
+                    uint64_t Q0, int n, bool windows) {
+    uint64_t best_q = Q0;
+    int best = scan_items(items, left, lim, best_q, true, nullptr);
+    if (n <= lim.K) return best_q;
+    auto offer = [&](uint64_t Q, int got) {
+        if (got > best) {
+            best = got;
+            best_q = Q;
+        }
+    };
+    const int w = lim.K - popc(Q0);
+    if (windows && w > 0 && w < 64) {
+        const int low = popc(Q0);
+        for (int a = low; a + w <= n; ++a) {
+            uint64_t Q = Q0 | (((uint64_t(1) << w) - 1) << a);
+            if (popc(Q) == lim.K) offer(Q, scan_items(items, left, lim, Q, false, nullptr));
+        }
+    }
+    uint64_t Q = Q0;
+    int got = scan_items(items, left, lim, Q, false, nullptr);
+    while (popc(Q) < lim.K) {
+        int step_got = -1;
+        uint64_t step_q = Q;
+        for (int q = 0; q < n; ++q) {
+            if (Q >> q & 1) continue;
+            uint64_t t = Q | uint64_t(1) << q;
+            const int g = scan_items(items, left, lim, t, false, nullptr);
+            if (g > step_got) {
+                step_got = g;
+                step_q = t;
+            }
+        }
+        Q = step_q;
+        got = step_got;
+    }
+    offer(Q, got);
+    return best_q;
+}
+
+// A group of items that run together under one set; `single`: an item that runs alone, outside any set.
+struct Cut {
+    uint64_t set = 0;
+    std::vector<int> members;
+    bool single = false;
+};
+
+// Cut the items into groups, each group's set taken in program order or, with `search`, by choose_set.
+std::vector<Cut> cut_items(const std::vector<ScanItem> &items, const ScanLimits &lim, uint64_t Q0, int n, bool windows,
+                           bool search) {
+    std::vector<int> left(items.size()), rest;
+    for (size_t i = 0; i < items.size(); ++i) left[i] = int(i);
+    std::vector<Cut> out;
+    while (!left.empty()) {
+        Cut c;
+        if (items[size_t(left.front())].fusable) {
+            c.set = Q0;
+            if (search) c.set = choose_set(items, left, lim, Q0, n, windows);
+            scan_items(items, left, lim, c.set, !search, &c.members);
+        }
+        if (c.members.empty()) {
+            // not fusable, or too wide for the room next to Q0
+            c.single = true;
+            c.members.push_back(left.front());
+        }
+        rest.clear();
+        std::set_difference(left.begin(), left.end(), c.members.begin(), c.members.end(), std::back_inserter(rest));
+        left.swap(rest);
+        out.push_back(std::move(c));
+    }
+    return out;
+}
+
+// The cut with fewer groups; program order where the search saves none (its groups are more even).
+std::vector<Cut> best_cut(const std::vector<ScanItem> &items, const ScanLimits &lim, uint64_t Q0, int n, bool windows) {
+    std::vector<Cut> plain = cut_items(items, lim, Q0, n, windows, false);
+    if (n <= lim.K || plain.size() < 3) return plain;
+    std::vector<Cut> found = cut_items(items, lim, Q0, n, windows, true);
+    return found.size() < plain.size() ? found : plain;
+}
+
+}  // namespace
+
+Schedule build_schedule(int n, int K, int c, const std::vector<DevOp> &ops, bool fuse, const std::vector<char> *no_fuse,
+                        const PassLimits &limits) {
     auto fusable_at = [&](int i) { return fusable(ops[i]) && !(no_fuse && (*no_fuse)[i]); };
     Schedule s;
     if (K > n) K = n;
@@ -86,13 +221,26 @@ Schedule build_schedule(int n, int K, int c, const std::vector<DevOp> &ops, bool
     if (K < 6) fuse = false;
     s.K = K;
     const int L = int(ops.size());
-    std::vector<char> done(L, 0);
-    int n_done = 0;
-    int first = 0;
     const uint64_t all = n >= 64 ? ~uint64_t(0) : ((uint64_t(1) << n) - 1);
-    while (n_done < L) {
-        while (first < L && done[first]) ++first;
-        if (!fuse || !fusable_at(first)) {
+    std::vector<ScanItem> items(static_cast<size_t>(L));
+    for (int i = 0; i < L; ++i) {
+        ScanItem &it = items[size_t(i)];
+        it.touch = touched(ops[i]);
+        it.dense = dense_targets(ops[i]);
+        it.slots = popc(uint64_t(ops[i].grad_mask));
+        it.entries = ops[i].mat_size * (1 + (limits.derivatives && ops[i].grad_mask ? ops[i].n_angles : 0));
+        it.fusable = fuse && fusable_at(i);
+    }
+    ScanLimits lim;
+    lim.K = K;
+    lim.max_items = kMaxPassOps;
+    lim.max_slots = kMaxPassSlots;
+    lim.max_entries = limits.max_entries;
+    lim.all = all;
+    for (const Cut &cut : best_cut(items, lim, (n <= K) ? all : ((uint64_t(1) << c) - 1), n, true)) {
+        const std::vector<int> &members = cut.members;
+        if (cut.single) {
+            const int first = members.front();
             Pass p;
             p.fused = 0;
             p.op_begin = first;
@@ -100,50 +248,9 @@ Schedule build_schedule(int n, int K, int c, const std::vector<DevOp> &ops, bool
             p.prog_op_begin = first;
             p.prog_op_end = first + 1;
             s.passes.push_back(p);
-            done[first] = 1;
-            ++n_done;
             continue;
         }
-        uint64_t Q = (n <= K) ? all : ((uint64_t(1) << c) - 1);
-        uint64_t blocked = 0;
-        std::vector<int> members;
-        int n_slots = 0;
-        for (int i = first; i < L && int(members.size()) < kMaxPassOps; ++i) {
-            if (done[i]) continue;
-            const DevOp &op = ops[i];
-            const uint64_t t = touched(op);
-            if (t & blocked) {
-                blocked |= t;
-                if ((blocked & all) == all) break;
-                continue;
-            }
-            if (!fusable_at(i)) {
-                blocked |= t;
-                continue;
-            }
-            const uint64_t need = dense_targets(op) & ~Q;
-            const int op_slots = popc(uint64_t(op.grad_mask));
-            if (popc(Q | need) <= K && n_slots + op_slots <= kMaxPassSlots) {
-                Q |= need;
-                n_slots += op_slots;
-                members.push_back(i);
-            } else {
-                blocked |= t;
-            }
-        }
-        if (members.empty()) {
-            // the first gate does not fit next to the contiguity bits: run it on its own
-            Pass p;
-            p.fused = 0;
-            p.op_begin = first;
-            p.op_end = first + 1;
-            p.prog_op_begin = first;
-            p.prog_op_end = first + 1;
-            s.passes.push_back(p);
-            done[first] = 1;
-            ++n_done;
-            continue;
-        }
+        uint64_t Q = cut.set;
         // pad the tile to exactly K qubits with the lowest free qubits
         for (int q = 0; q < n && popc(Q) < K; ++q) Q |= uint64_t(1) << q;
         Pass p;
@@ -193,13 +300,11 @@ Schedule build_schedule(int n, int K, int c, const std::vector<DevOp> &ops, bool
                     if (op.grad_mask >> a & 1) s.slot_map.push_back(op.slot0 + r++);
             }
             s.pass_ops.push_back(po);
-            done[i] = 1;
-            ++n_done;
         }
         p.op_end = int(s.pass_ops.size());
         p.n_slots = int(s.slot_map.size()) - p.slot_begin;
-        p.prog_op_begin = members.empty() ? first : members.front();
-        p.prog_op_end = members.empty() ? first : members.back() + 1;
+        p.prog_op_begin = members.front();
+        p.prog_op_end = members.back() + 1;
         s.passes.push_back(p);
     }
     return s;
@@ -308,29 +413,23 @@ void build_stages(Schedule &s, const std::vector<DevOp> &ops, int reg_bits, int 
         const int sop_begin = int(stage_ops.size());
         int mtab = 0;
         const int npo = p.op_end - p.op_begin;
-        std::vector<char> done(npo, 0);
-        int n_done = 0;
-        while (n_done < npo) {
-            uint32_t R = 0, blocked = 0;
-            std::vector<int> members;
-            for (int i = 0; i < npo; ++i) {
-                if (done[i]) continue;
-                const PassOp &po = s.pass_ops[p.op_begin + i];
-                uint32_t touch = po.lctrl, dense = 0;
-                for (int k = 0; k < po.m; ++k)
-                    if (po.lt[k] >= 0) touch |= 1u << po.lt[k];
-                if (po.kind == KIND_DENSE) dense = touch & ~po.lctrl;
-                if (touch & blocked) {
-                    blocked |= touch;
-                    continue;
-                }
-                if (popc(R | dense) <= RB) {
-                    R |= dense;
-                    members.push_back(i);
-                } else {
-                    blocked |= touch;
-                }
-            }
+        std::vector<ScanItem> items(static_cast<size_t>(npo));
+        for (int i = 0; i < npo; ++i) {
+            const PassOp &po = s.pass_ops[p.op_begin + i];
+            ScanItem &it = items[size_t(i)];
+            it.touch = po.lctrl;
+            for (int k = 0; k < po.m; ++k)
+                if (po.lt[k] >= 0) it.touch |= 1u << po.lt[k];
+            if (po.kind == KIND_DENSE) it.dense = it.touch & ~uint64_t(po.lctrl);
+        }
+        ScanLimits lim;
+        lim.K = RB;
+        lim.all = (uint64_t(1) << K) - 1;
+        for (const Cut &cut : best_cut(items, lim, 0, K, false)) {
+            const std::vector<int> &members = cut.members;
+            // keep only the bits that a member needs: the rest is padded below
+            uint32_t R = 0;
+            for (int i : members) R |= uint32_t(items[size_t(i)].dense);
             // padding: add local bits so that the thread bits keep one bit of every residue class
             auto thread_residue_count = [&](uint32_t Rm, int r) {
                 int cnt = 0;
@@ -388,7 +487,7 @@ void build_stages(Schedule &s, const std::vector<DevOp> &ops, int reg_bits, int 
                 so.n_angles = dop.grad_mask ? dop.n_angles : 0;
                 so.mat_size = dop.mat_size;
                 so.moff = mtab;
-                so.mcount = dop.mat_size * (1 + so.n_angles);
+                so.mcount = forward ? dop.mat_size : dop.mat_size * (1 + so.n_angles);   // a forward pass reads M alone
                 so.msrc = dop.mat_off;
                 so.msrc_ps = dop.per_sample;
                 mtab += so.mcount;
@@ -429,8 +528,6 @@ void build_stages(Schedule &s, const std::vector<DevOp> &ops, int reg_bits, int 
                 }
                 assign_codes(so);
                 stage_ops.push_back(so);
-                done[i] = 1;
-                ++n_done;
             }
             sd.op_end = int(stage_ops.size()) - sop_begin;
             stages.push_back(sd);
