@@ -17,8 +17,8 @@ CSRC = os.path.join(HERE, 'csrc')
 INCLUDE = os.path.join(os.path.dirname(HERE), 'include')
 LIB = os.path.join(HERE, 'libmqb200.so')
 FUSED = ['fused_fwd_c64.cu', 'fused_fwd_c128.cu', 'fused_bwd_c64.cu', 'fused_bwd_c128.cu']
-SOURCES = ['kernels.cu', *FUSED, 'capi.cpp', 'scheduler.cpp', 'noalloc.cu', 'jit.cpp']
-HEADERS = ['kernels.cuh', 'mqb_internal.h', 'mqb_gate_ids.h', 'fused_impl.cuh', 'regops.cuh', 'regmath.cuh',
+SOURCES = ['kernels.cu', 'small.cu', *FUSED, 'capi.cpp', 'scheduler.cpp', 'noalloc.cu', 'jit.cpp']
+HEADERS = ['kernels.cuh', 'small.h', 'mqb_internal.h', 'mqb_gate_ids.h', 'fused_impl.cuh', 'regops.cuh', 'regmath.cuh',
            'tile.cuh', 'jit_abi.h', 'jit.h', 'pipe.cuh']
 # headers compiled again at run time by NVRTC for the generated pass kernels (embedded as text)
 JIT_HEADERS = [('kJitRegmath', 'regmath.cuh'), ('kJitTile', 'tile.cuh'), ('kJitAbi', 'jit_abi.h'),
@@ -81,7 +81,7 @@ def build(force=False, verbose=False):
             f.write(text)
 
     compiles = [[_nvcc(), *ARCH, '-lineinfo', *common, '-c', os.path.join(CSRC, f), '-o', obj(f)]
-                for f in ('kernels.cu', *FUSED, 'noalloc.cu')]
+                for f in ('kernels.cu', 'small.cu', *FUSED, 'noalloc.cu')]
     compiles.append([_nvcc(), *ARCH, '-lineinfo', *common, '-x', 'cu', '-c', os.path.join(CSRC, 'capi.cpp'),
                      '-o', obj('capi.cpp')])
     compiles.append([_nvcc(), *common, '-x', 'c++', '-c', os.path.join(CSRC, 'scheduler.cpp'),

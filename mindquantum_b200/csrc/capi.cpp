@@ -20,6 +20,7 @@
 
 #include "jit.h"
 #include "kernels.cuh"
+#include "small.h"
 
 namespace {
 
@@ -192,7 +193,10 @@ struct SchedDev {
     std::mutex jit_mu;
     std::vector<const void *> jit_fwd;                // generated forward kernel of every pass
     std::map<int, std::vector<const void *>> jit_bwd; // generated backward kernels, by lambdas
+    SmallOp *d_small = nullptr;                       // the gates in execution order, when the block-per-sample kernel runs them
+    size_t small_smem = 0;                            // its shared memory (0: the tile kernels run)
     ~SchedDev() {
+        cudaFree(d_small);
         cudaFree(d_jmt);
         cudaFree(d_f_jmt);
         cudaFree(s.d_pass_ops);
@@ -212,6 +216,7 @@ struct mqb_program {
     mqb_gate_desc *d_descs = nullptr;
     mqb_param_term *d_terms = nullptr;
     void *d_cpool = nullptr;
+    int64_t n_pool = 0;        // complex entries of the constant pool
     int64_t per_sample = 0;    // complex entries per sample
     int64_t custom_entries = 0;
     int n_slots = 0;
@@ -277,6 +282,56 @@ static PassLimits pass_limits(const mqb_program &p, int K, int reg_bits, int n_h
     return lim;
 }
 
+static int norm_stride(int passes) { return std::max(1, int(std::ceil(std::sqrt(double(passes))))); }
+
+// Largest register of the block-per-sample kernel.  One evaluation of a 3-layer ansatz (2 launches
+// against 7 and more): at 10 qubits it and the tile kernels both hide behind the host's 260 us per call, at 11
+// one sample with 4 Hamiltonians takes 409 us here and 400 there, at 12 724 against 505.
+constexpr int kSmallMaxQubits = 10;
+// Registers up to this size run here at any batch, larger ones up to two samples per SM: with 1024
+// samples, 8 qubits take 376 (complex64, 4 Hamiltonians) and 269 us (complex128, one) against 341 and 288
+// of the tile kernels, 9 qubits 475 against 321, 10 qubits 1030 against 429.
+constexpr int kSmallAnyBatchQubits = 8;
+
+// The block-per-sample kernel's gate list, in the schedule's execution order, when it can run the
+// program: gates of at most two targets, unitary where a gradient undoes them, everything in one
+// block's shared memory.  Callers that force a kernel family (jit, tile_bits, fuse) get that one.
+static void plan_small(const mqb_program &p, SchedDev &sd, int n_hams) {
+    if (!p.fuse || p.jit != 0 || p.tile_bits != 0 || p.n > kSmallMaxQubits || p.ops.empty()) return;
+    if (n_hams > 0 && p.nonunitary) return;
+    for (const DevOp &op : p.ops)
+        if (op.kind == KIND_RPS || op.m > kMaxFusedM) return;
+    const size_t smem = small_smem(p.n, int(p.elem()), n_hams, int(p.ops.size()), p.per_sample + p.n_pool, n_hams ? p.n_slots : 0);
+    if (!smem) return;
+    std::vector<SmallOp> v;
+    const int P = int(sd.s.passes.size()), sn = norm_stride(P);
+    for (int q = 0; q < P; ++q) {
+        const Pass &ps = sd.s.passes[size_t(q)];
+        for (int i = ps.op_begin; i < ps.op_end; ++i) {
+            const DevOp &op = p.ops[size_t(ps.fused ? sd.s.pass_ops[size_t(i)].op : i)];
+            SmallOp so{};
+            so.kind = op.kind;
+            so.m = op.m;
+            so.sub = op.sub;
+            so.t0 = op.tq[0];
+            so.t1 = op.m > 1 ? op.tq[1] : 0;
+            so.ctrl = uint32_t(op.ctrl);
+            so.moff = int32_t(op.per_sample ? op.mat_off : p.per_sample + op.mat_off);
+            so.doff = op.dmat_off;
+            so.mat_size = op.mat_size;
+            so.grad_mask = op.grad_mask;
+            so.slot0 = op.slot0;
+            const int done = q + 1;
+            // norm checks as grad_layout places them: after pass `done`, and of the state before pass q
+            if (i + 1 == ps.op_end && (done % sn == 0 || done == P)) so.check |= 1;
+            if (i == ps.op_begin && q % sn == 0) so.check |= q << 1;
+            v.push_back(so);
+        }
+    }
+    sd.d_small = upload(v);
+    sd.small_smem = smem;
+}
+
 static std::unique_ptr<SchedDev> make_sched(const mqb_program &p, int K, bool fuse, int reg_bits, int n_hams) {
     auto sd = std::make_unique<SchedDev>();
     // the register kernels need 2^5..2^8 threads of 2^reg_bits amplitudes: smaller registers use
@@ -294,6 +349,7 @@ static std::unique_ptr<SchedDev> make_sched(const mqb_program &p, int K, bool fu
     sd->s.d_f_stage_ops = upload(sd->s.f_stage_ops);
     sd->d_jmt = upload(jit_mtab(sd->s.stage_ops));
     sd->d_f_jmt = upload(jit_mtab(sd->s.f_stage_ops));
+    plan_small(p, *sd, n_hams);
     return sd;
 }
 
@@ -399,6 +455,28 @@ static void run_matgen(const mqb_program &p, const double *params, int64_t param
     ck(launch_matgen<R>(m, st), "matgen");
 }
 
+// Whether a call runs the block-per-sample kernel: the schedule has it, and the tile kernels either cannot
+// fuse this register or are not the faster ones at this batch.
+static bool runs_small(const mqb_program &p, const SchedDev &sd, int64_t batch) {
+    if (!sd.small_smem) return false;
+    const bool tiles = std::any_of(sd.s.passes.begin(), sd.s.passes.end(), [](const Pass &ps) { return ps.fused != 0; });
+    return !tiles || p.n <= kSmallAnyBatchQubits || batch <= 2 * int64_t(sm_count_cached());
+}
+
+template <typename R>
+static SmallArgs<R> small_args(const mqb_program &p, const SchedDev &sd, const cplx<R> *mats, int64_t batch) {
+    SmallArgs<R> a{};
+    a.n = p.n;
+    a.n_ops = int(p.ops.size());
+    a.ops = sd.d_small;
+    a.mats = mats;
+    a.mats_stride = p.per_sample;
+    a.cpool = static_cast<const cplx<R> *>(p.d_cpool);
+    a.n_pool = int(p.n_pool);
+    a.batch = batch;
+    return a;
+}
+
 template <typename R>
 static void apply_impl(mqb_program &p, void *states, int64_t batch, const double *params, int64_t param_stride,
                        const double *custom, void *ws, size_t ws_bytes, cudaStream_t st) {
@@ -408,6 +486,15 @@ static void apply_impl(mqb_program &p, void *states, int64_t batch, const double
     run_matgen<R>(p, params, param_stride, custom, batch, mats, st);
     cplx<R> *s = static_cast<cplx<R> *>(states);
     SchedDev &sd = *p.apply_sched;
+    if (runs_small(p, sd, batch)) {
+        SmallArgs<R> a = small_args<R>(p, sd, mats, batch);
+        a.src = s;
+        a.src_stride = int64_t(1) << p.n;
+        a.dst = s;
+        TimeScope ts(TK_FWD, st);
+        ck(launch_small<R>(a, sd.small_smem, st), "small register");
+        return;
+    }
     const auto *jk = jit_forward(p, sd);
     for (size_t i = 0; i < sd.s.passes.size(); ++i)
         run_forward_pass<R>(p, sd, i, jk ? (*jk)[i] : nullptr, mats, s, int64_t(1) << p.n, s, batch, st);
@@ -534,7 +621,7 @@ static GradLayout grad_layout(const mqb_program &p, const Schedule &s, int64_t b
     if (P == 0) L.need_w = true;
     if (p.precision == MQB_PREC_C64 && P > 0) {
         // every ceil(sqrt(P)) passes (and the last state of the forward sweep)
-        const int sn = std::max(1, int(std::ceil(std::sqrt(double(P)))));
+        const int sn = norm_stride(P);
         for (int q = 1; q <= P; ++q)
             if (q % sn == 0 || q == P) L.norm_fwd.push_back(q);
         for (int q = P - 1; q >= 1; --q)
@@ -580,6 +667,31 @@ static void grad_impl(mqb_program &p, const mqb_hamiltonian *const *hams, int n_
     const int sm = sm_count_cached();
     const V *cpool = static_cast<const V *>(p.d_cpool);
 
+    if (runs_small(p, sd, batch) && std::none_of(hams, hams + (lam_in ? 0 : n_hams), [](const mqb_hamiltonian *h) { return h->csr; })) {
+        run_matgen<R>(p, params, param_stride, custom, batch, mats, st);
+        SmallArgs<R> a = small_args<R>(p, sd, mats, batch);
+        a.src = static_cast<const V *>(init);
+        a.src_stride = init_batched ? dim : 0;
+        a.n_hams = n_hams;
+        for (int h = 0; h < n_hams && !lam_in; ++h)
+            a.ham[h] = SmallHam{hams[h]->d_classes, hams[h]->d_terms, int(hams[h]->classes.size())};
+        a.lam_in = static_cast<const V *>(lam_in);
+        a.lam_stride = lam_batched ? dim : 0;
+        a.f = f;
+        a.grad = grad;
+        a.n_params = p.n_params;
+        a.n_slots = p.n_slots;
+        a.csr_ptr = p.d_csr_ptr;
+        a.csr_slot = p.d_csr_slot;
+        a.csr_coeff = p.d_csr_coeff;
+        a.scale = lam_in ? 1.0 : 2.0;
+        // the sweep rebuilds every state; the checks it keeps are those of this stride's layout
+        a.norms = L.norms ? reinterpret_cast<double *>(ck0 + L.ckpt) : nullptr;
+        a.ckpt_stride = stride;
+        TimeScope ts(TK_BWD, st);
+        ck(launch_small<R>(a, sd.small_smem, st), "small register gradient");
+        return;
+    }
     ck(cudaMemsetAsync(gslots, 0, L.gslots, st), "memset");
     if (f) ck(cudaMemsetAsync(f, 0, sizeof(double) * 2 * n_hams * batch, st), "memset");
     // norm checks: <psi|psi> in FP64 per sample, [check][batch][re, im]
@@ -949,6 +1061,7 @@ int mqb_program_create(int n_qubits, int precision, const mqb_gate_desc *gates, 
         p->d_ops = upload(p->ops);
         p->d_descs = upload(p->descs);
         p->d_terms = upload(std::vector<mqb_param_term>(terms, terms + n_terms));
+        p->n_pool = int64_t(pool.size());
         if (!pool.empty()) {
             if (precision == MQB_PREC_C64) {
                 std::vector<float2> v;

@@ -1,0 +1,64 @@
+// Registers small enough for one block's shared memory: a whole evaluation in one launch (small.cu).
+#ifndef MQB_SMALL_H_
+#define MQB_SMALL_H_
+
+#include "kernels.cuh"
+
+namespace mqb {
+
+constexpr int kSmallMaxHams = 4;
+
+// One gate of the small-register kernel, in execution order.
+struct SmallOp {
+    int32_t kind, m, sub;        // OpKind, targets, DenseSub
+    int32_t t0, t1;              // target qubits (matrix bits 0 and 1)
+    uint32_t ctrl;               // control mask
+    int32_t moff;                // M in the block's matrix table: the per-sample block, then the constant pool
+    int32_t doff;                // dM_a at doff + a * mat_size
+    int32_t mat_size;
+    int32_t grad_mask, slot0;    // gradient angles (0: none) and the slot of the first one
+    int32_t check;               // bit 0: norm check after the gate; bits 1..: pass q whose start the gate is,
+                                 // for the check of the state before it in the backward sweep (0: none)
+};
+
+struct SmallHam {
+    const HamClass *classes;
+    const HamTerm *terms;
+    int n_classes;
+};
+
+template <typename R>
+struct SmallArgs {
+    int n, n_ops;
+    const SmallOp *ops;
+    const cplx<R> *mats;         // per-sample matrices
+    int64_t mats_stride;
+    const cplx<R> *cpool;
+    int n_pool;
+    const cplx<R> *src;          // nullptr: |0...0>
+    int64_t src_stride;
+    cplx<R> *dst;                // apply: the final state; gradient: nullptr
+    int64_t batch;
+    // gradient
+    int n_hams;
+    SmallHam ham[kSmallMaxHams];
+    const cplx<R> *lam_in;       // lambda from the caller instead of the Hamiltonians (n_hams = 1)
+    int64_t lam_stride;
+    double *f;                   // [batch][n_hams][2]
+    double *grad;                // [batch][n_hams][n_params]
+    int n_params, n_slots;
+    const int32_t *csr_ptr, *csr_slot;
+    const double *csr_coeff;
+    double scale;
+    double *norms;               // [check][batch][2], or nullptr (no checks)
+    int ckpt_stride;             // the states the caller's layout counts as stored have no backward check
+};
+
+// Shared memory of a block; 0 when the evaluation does not fit the kernel.
+size_t small_smem(int n, int elem_bytes, int n_hams, int n_ops, int64_t table_entries, int n_slots);
+template <typename R>
+cudaError_t launch_small(const SmallArgs<R> &a, size_t smem, cudaStream_t s);
+
+}  // namespace mqb
+
+#endif
