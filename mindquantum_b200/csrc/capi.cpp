@@ -249,14 +249,14 @@ JitBlock::~JitBlock() { t_jit_blocked = prev_; }
 
 static std::vector<JitMtab> jit_mtab(const std::vector<StageOp> &v) {
     std::vector<JitMtab> o(v.size());
-    for (size_t i = 0; i < v.size(); ++i) o[i] = JitMtab{v[i].moff, v[i].mcount, (long long)v[i].msrc, v[i].msrc_ps, 0};
+    for (size_t i = 0; i < v.size(); ++i) o[i] = JitMtab{v[i].moff, v[i].mcount, (long long)v[i].msrc, v[i].msrc_ps, v[i].phase & ~kPhaseUnitary};
     return o;
 }
 
 static const std::vector<const void *> *jit_forward(const mqb_program &p, SchedDev &sd) {
     if (!p.use_jit() || t_jit_blocked || sd.s.passes.empty()) return nullptr;
     std::lock_guard<std::mutex> lk(sd.jit_mu);
-    if (sd.jit_fwd.empty()) sd.jit_fwd = jit_forward_kernels(sd.s, p.precision);
+    if (sd.jit_fwd.empty()) sd.jit_fwd = jit_forward_kernels(sd.s, p.precision, p.ops);
     return &sd.jit_fwd;
 }
 
@@ -273,7 +273,8 @@ static const std::vector<const void *> *jit_backward(const mqb_program &p, Sched
 // for a table.  n_hams = 0: a forward schedule.
 static PassLimits pass_limits(const mqb_program &p, int K, int reg_bits, int n_hams) {
     const int64_t buf = (int64_t(1) << K) * int64_t(p.elem()) * (1 + n_hams);
-    const int64_t slots = int64_t(1 << std::max(0, K - reg_bits - 5)) * kMaxPassSlots * n_hams * int64_t(sizeof(double));
+    const int64_t warps = int64_t(1) << std::max(0, K - reg_bits - 5);
+    const int64_t slots = n_hams ? warps * (kMaxPassSlots * n_hams * int64_t(sizeof(double)) + 512) : 0;
     auto table = [&](int buffers) { return ((int64_t(227) << 10) - 256 - buffers * buf) / 2 - slots; };
     const int64_t bytes = table(3) >= 8192 ? table(3) : table(2);
     PassLimits lim;
@@ -340,7 +341,7 @@ static std::unique_ptr<SchedDev> make_sched(const mqb_program &p, int K, bool fu
     sd->s = build_schedule(p.n, K, contiguity_bits(p.precision), p.ops, fuse, &p.no_fuse,
                            pass_limits(p, K, reg_bits, n_hams));
     build_stages(sd->s, p.ops, reg_bits, p.precision, false);
-    build_stages(sd->s, p.ops, fwd_reg_bits(p.precision), p.precision, true);
+    build_stages(sd->s, p.ops, p.use_jit() ? jit_fwd_reg_bits(p.precision) : fwd_reg_bits(p.precision), p.precision, true);
     sd->s.d_pass_ops = upload(sd->s.pass_ops);
     sd->s.d_slot_map = upload(sd->s.slot_map);
     sd->s.d_stages = upload(sd->s.stages);
@@ -876,6 +877,15 @@ static DevOp basic_op(const mqb_gate_desc &d, int k, int n_qubits, const mqb_par
         op.per_sample = 0;
         op.n_angles = 0;
         op.grad_mask = 0;
+        op.unitary = 1;
+        for (int r = 0; r < dimm; ++r)
+            for (int q = 0; q < dimm; ++q) {
+                std::complex<double> dot = r == q ? -1.0 : 0.0;   // (M M^dag - 1)_rq
+                for (int c = 0; c < dimm; ++c)
+                    dot += std::complex<double>(m[2 * (r * dimm + c)], m[2 * (r * dimm + c) + 1]) *
+                           std::complex<double>(m[2 * (q * dimm + c)], -m[2 * (q * dimm + c) + 1]);
+                if (std::abs(dot) > 1e-12) op.unitary = 0;
+            }
         op.kind = diag ? KIND_DIAG : KIND_DENSE;
         op.mat_size = diag ? dimm : dimm * dimm;
         op.sub = SUB_GENERIC;
@@ -914,6 +924,7 @@ static DevOp basic_op(const mqb_gate_desc &d, int k, int n_qubits, const mqb_par
         if (d.gate_id == GID_RY) op.sub = SUB_REAL;   // RY and its derivative are real matrices
         if (d.gate_id == GID_RX) op.sub = SUB_RXL;    // RX: real diagonal, imaginary off-diagonal
     }
+    op.unitary = d.gate_id != GID_CUSTOM;
     const int expect_obj =
         (d.gate_id == GID_RZZ || (d.gate_id >= GID_RXX && d.gate_id <= GID_SWAPALPHA) || d.gate_id == GID_FSIM) ? 2 : 1;
     if (d.gate_id != GID_CUSTOM && d.n_obj != expect_obj)
@@ -1085,7 +1096,7 @@ int mqb_program_create(int n_qubits, int precision, const mqb_gate_desc *gates, 
         p->d_csr_ptr = upload(ptr);
         p->d_csr_slot = upload(slot);
         p->d_csr_coeff = upload(coeff);
-        const int rb = fwd_reg_bits(precision);
+        const int rb = p->use_jit() ? jit_fwd_reg_bits(precision) : fwd_reg_bits(precision);
         p->apply_sched = make_sched(*p, tile_bits_for(*p, rb), p->fuse != 0, rb, 0);
         *out = p.release();
     });
@@ -1099,7 +1110,8 @@ int mqb_plan_schedule(int n_qubits, int precision, const mqb_gate_desc *gates, i
         std::vector<DevOp> ops;
         for (int k = 0; k < n_gates; ++k)
             ops.push_back(basic_op(gates[k], k, n_qubits, nullptr, 0, 0, const_matrices, n_const_entries));
-        const int rb = fwd_reg_bits(precision);
+        // the register bits mqb_program_create takes by default (generated kernels from 18 qubits on)
+        const int rb = n_qubits >= 18 && tile_bits == 0 ? jit_fwd_reg_bits(precision) : fwd_reg_bits(precision);
         int K = std::min(n_qubits, rb + 8);
         if (tile_bits > 0) K = std::min(n_qubits, std::max(rb + 5, tile_bits));
         Schedule s = build_schedule(n_qubits, K, contiguity_bits(precision), ops, fuse != 0 && K >= rb + 5);
@@ -1142,12 +1154,12 @@ int mqb_jit_check(int n_qubits, int precision, const mqb_gate_desc *gates, int n
             }
             ops.push_back(op);
         }
-        const int rb = n_hams ? bwd_reg_bits(precision, n_hams) : fwd_reg_bits(precision);
+        const int rb = n_hams ? bwd_reg_bits(precision, n_hams) : jit_fwd_reg_bits(precision);
         int K = std::min(n_qubits, rb + 8);
         if (tile_bits > 0) K = std::min(n_qubits, std::max(rb + 5, tile_bits));
         Schedule s = build_schedule(n_qubits, K, contiguity_bits(precision), ops, K >= rb + 5);
         build_stages(s, ops, rb, precision, false);
-        build_stages(s, ops, fwd_reg_bits(precision), precision, true);
+        build_stages(s, ops, jit_fwd_reg_bits(precision), precision, true);
         *n_kernels = jit_compile_check(s, precision, n_hams, ops);
     });
 }

@@ -22,6 +22,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <sstream>
@@ -31,11 +32,12 @@
 
 namespace mqb {
 
-// Header texts for NVRTC, embedded at build time from regmath.cuh, tile.cuh, jit_abi.h and pipe.cuh.
+// Header texts for NVRTC, embedded at build time from regmath.cuh, tile.cuh, jit_abi.h, pipe.cuh and phasemath.cuh.
 extern const char *const kJitRegmath;
 extern const char *const kJitTile;
 extern const char *const kJitAbi;
 extern const char *const kJitPipe;
+extern const char *const kJitPhase;
 
 namespace {
 
@@ -179,7 +181,30 @@ std::string lit(double x) {
     return o.str();
 }
 
-void emit_backward_op(std::ostringstream &o, const StageOp &so, int NH, int gid) {
+// Gradient partials of an adjoint kernel.  A thread's partial of one (angle, Hamiltonian) is a row of its
+// warp's shared scratch; every kRowBatch rows the warp adds them up together (pipe::rows_flush_as): 5
+// instructions per row instead of 16 for a shuffle tree per partial, which was 30 to 40 % of the adjoint passes
+// (26-qubit ansatz, batch 2: 36.6 ms with the trees, 25.9 with no reduction at all).
+// Rows come in the order the kernel makes them; `order` maps them to pass-local slots.
+int row_batch(int precision) { return precision == MQB_PREC_C64 ? 4 : 2; }
+
+struct Rows {
+    int batch = 4, NH = 1;
+    std::vector<int> order;   // row -> lslot * NH + h
+
+    void flush(std::ostringstream &o) const {
+        const int n = int(order.size()) % batch == 0 ? batch : int(order.size()) % batch;
+        o << "    pipe::rows_flush_as<R>(scr, wrow + " << int(order.size()) - n << ", " << n << ", lane);\n";
+    }
+    // the partial `expr` of slot lslot and Hamiltonian h
+    void put(std::ostringstream &o, const std::string &expr, int lslot, int h) {
+        o << "      pipe::row_put(scr, " << int(order.size()) % batch << ", lane, " << expr << ");\n";
+        order.push_back(lslot * NH + h);
+        if (int(order.size()) % batch == 0) flush(o);
+    }
+};
+
+void emit_backward_op(std::ostringstream &o, const StageOp &so, int NH, int gid, Rows &rows) {
     const std::string on = on_expr(so);
     const bool cond = !on.empty();
     const int M = so.moff;
@@ -194,10 +219,8 @@ void emit_backward_op(std::ostringstream &o, const StageOp &so, int NH, int gid)
     auto sel = [&](const std::string &val, const std::string &id) { return cond ? "(on ? " + val + " : " + id + ")" : val; };
     const std::string one = "cval<V>(1, 0)", zero = "cval<V>(0, 0)";
     auto dm = [&](int a, int e) { return mt(M + ms * (1 + a) + e); };
-    const std::vector<double> pw = (G == 1) ? phase_weights(gid) : std::vector<double>();
     const bool gen_ry = G == 1 && gid == GID_RY && so.kind == SK_REAL1;
     const bool gen_rx = G == 1 && gid == GID_RX && so.kind == SK_RXL1;
-    const bool gen_diag = !pw.empty() && (so.kind == SK_DIAG1 || so.kind == SK_DIAG2);
     const bool gen_u3 = G != 0 && gid == GID_U3 && so.kind == SK_DENSE1;
     auto wsel = [&](const std::string &w) { return cond ? "(on ? " + w + " : R(0))" : w; };
     if (gen_u3) {
@@ -216,36 +239,6 @@ void emit_backward_op(std::ostringstream &o, const StageOp &so, int NH, int gid)
     } else if (gen_rx) {
         o << "      jbg_rx<V, RB, NH, " << so.p0 << ", " << CM << ">(v, l, " << sel(mt(M) + ".x", "R(1)") << ", "
           << sel("-" + mt(M + 1) + ".y", "R(0)") << ", " << wsel("R(0.5)") << ", acc);\n";
-    } else if (gen_diag) {
-        const bool two = so.kind == SK_DIAG2;
-        const bool in0 = so.dsrc[0] == 0, in1 = two && so.dsrc[1] == 0;
-        auto c = [&](const std::string &idx) { return sel("cconj(mt[" + std::to_string(M) + " + " + idx + "])", one); };
-        if (!two && in0) {
-            o << "      jbg_diag1<V, RB, NH, " << so.dval[0] << ", " << CM << ">(v, l, " << c("0") << ", " << c("1")
-              << ", " << wsel(lit(pw[0])) << ", " << wsel(lit(pw[1])) << ", acc);\n";
-        } else if (two && in0 && in1) {
-            o << "      const V c[4] = {" << c("0") << ", " << c("1") << ", " << c("2") << ", " << c("3") << "};\n";
-            o << "      const R w[4] = {" << wsel(lit(pw[0])) << ", " << wsel(lit(pw[1])) << ", " << wsel(lit(pw[2]))
-              << ", " << wsel(lit(pw[3])) << "};\n";
-            o << "      jbg_diag2<V, RB, NH, " << so.dval[0] << ", " << so.dval[1] << ", " << CM << ">(v, l, c, w, acc);\n";
-        } else if (two && (in0 || in1)) {
-            const int k = in0 ? 0 : 1;
-            o << "      const int b = " << off_bit_expr(so.dsrc[1 - k], so.dval[1 - k]) << ";\n";
-            if (k == 0) o << "      const int i0 = b << 1, i1 = 1 | (b << 1);\n";
-            else o << "      const int i0 = b, i1 = 2 | b;\n";
-            // weights of the register bit's two values, picked by the other target's bit (selects, no indexing)
-            const std::string w_lo = k == 0 ? "(b ? " + lit(pw[2]) + " : " + lit(pw[0]) + ")" : "(b ? " + lit(pw[1]) + " : " + lit(pw[0]) + ")";
-            const std::string w_hi = k == 0 ? "(b ? " + lit(pw[3]) + " : " + lit(pw[1]) + ")" : "(b ? " + lit(pw[3]) + " : " + lit(pw[2]) + ")";
-            o << "      jbg_diag1<V, RB, NH, " << so.dval[k] << ", " << CM << ">(v, l, " << c("i0") << ", " << c("i1")
-              << ", " << wsel(w_lo) << ", " << wsel(w_hi) << ", acc);\n";
-        } else {
-            o << "      const int r = " << off_bit_expr(so.dsrc[0], so.dval[0]) << " | ("
-              << off_bit_expr(two ? so.dsrc[1] : 3, so.dval[1]) << " << 1);\n";
-            const std::string w_r = pw.size() > 2 ? "(r == 0 ? " + lit(pw[0]) + " : r == 1 ? " + lit(pw[1]) + " : r == 2 ? " +
-                                                        lit(pw[2]) + " : " + lit(pw[3]) + ")"
-                                                  : "(r ? " + lit(pw[1]) + " : " + lit(pw[0]) + ")";
-            o << "      jbg_scale<V, RB, NH, " << CM << ">(v, l, " << c("r") << ", " << wsel(w_r) << ", acc);\n";
-        }
     } else
     switch (so.kind) {
         case SK_DENSE1:
@@ -318,244 +311,319 @@ void emit_backward_op(std::ostringstream &o, const StageOp &so, int NH, int gid)
         int r = 0;
         for (int a = 0; a < 3; ++a) {
             if (!((G >> a) & 1)) continue;
-            o << "      for (int h = 0; h < NH; ++h) {\n"
-              << "        const double x = double(warp_sum_acc(acc[" << a << "][h]));\n"
-              << "        if (lane == 0) wacc[(warp * NLS + " << (so.lslot + r) << ") * NH + h] += x;\n"
-              << "      }\n";
+            for (int h = 0; h < NH; ++h)
+                rows.put(o, "acc[" + std::to_string(a) + "][" + std::to_string(h) + "]", so.lslot + r, h);
             ++r;
         }
     }
     o << "    }\n";
 }
 
-// ------------------------------------------------------------------ runs of diagonal gates
-// Consecutive diagonal gates of a stage commute; their product is applied as one per-amplitude
-// factor.  Factors of targets off the registers are one scalar per thread, single-target factors
-// on register P are a pair (d0, d1) per thread, so a per-thread table over the register bits
-// carrying such factors costs about two complex products per amplitude for the whole run,
-// after which the run is one complex product per amplitude.  Two-target and register-controlled
-// factors are multiplied in per amplitude.  In the adjoint, Im(conj(lambda) psi) is the same at
-// every point of the run (a common unit-modulus diagonal cancels), so all gradients of the run
-// come from sums of it over the thread's amplitudes, split by the bits their weights depend on.
+// ------------------------------------------------------------------ diagonal gates of known unitaries
+// Consecutive diagonal gates of a stage commute, and most of their work can be taken out of the
+// per-amplitude path:
+//   * A pair (d0, d1) on a register bit is d0 times (1, r) with r = d1 / d0 (kept in the matrix table): only the amplitudes with
+//     the bit set are multiplied, a run of k such gates by a table of 2^k - 1 products (a ZZ pair the same way,
+//     by the parity of its two bits).
+//   * What is the same for all of a thread's amplitudes, a gate whose targets are off the registers
+//     or a taken-out d0, commutes with everything else the stage does to the registers: such factors
+//     collect in one scalar `sc` per thread, applied once at the end of the stage.  Factors that are the
+//     same for every thread (d0 of an uncontrolled gate) wait for the end of the pass (`ph`, made with the table).
+//   * In the adjoint, the sum S of Im(conj(lambda) psi) over a thread's amplitudes does not change under
+//     what the stage does to both states, so it is computed once per stage; a gate's gradient is then
+//     w0 S + (w1 - w0) SB with SB the sum over the amplitudes its bit selects, and a gate off
+//     the registers needs no sums at all.
+// The 26-qubit, 12-layer ansatz has 104 runs of such gates in its 63 adjoint stages.
+
+// State of the stage that is being written.
+struct StageCtx {
+    bool sc = false;   // `sc` carries a factor
+    bool S = false;    // `S` holds the thread's sums
+    int id = 0;
+};
 
 bool diag_op(const StageOp &so) { return so.kind == SK_DIAG1 || so.kind == SK_DIAG2; }
 
-// Gates a run may hold in the adjoint: no gradient, or a generator-form gradient.
-bool run_ok_backward(const StageOp &so, int gid) {
-    if (!diag_op(so)) return false;
+// Gates a run may hold: diagonal, unitary, and (adjoint) no gradient or a generator-form one.
+bool phase_op(const StageOp &so, int gid, bool adj) {
+    if (!diag_op(so) || !(so.phase & kPhaseUnitary)) return false;
     const int G = so.n_angles ? so.grad_mask : 0;
-    return G == 0 || (G == 1 && !phase_weights(gid).empty());
+    return !adj || G == 0 || (G == 1 && !phase_weights(gid).empty());
 }
 
-struct RunPlan {
-    std::vector<int> bits;   // register positions carrying per-thread factor pairs
-};
+// Whether the op leaves a factor for the end of its pass (pipe::pass_phase).
+bool leaves_factor(const StageOp &so) { return (so.phase & kPhaseKind) == kPhaseUniform || so.phase >> kPhaseNormShift; }
 
-enum DiagShape { DS_OFF, DS_REG1, DS_REGOFF, DS_OTHER };
-DiagShape diag_shape(const StageOp &so) {
+// Whether the thread's S survives the op: unitary on its registers.
+bool keeps_sums(const StageOp &so) { return so.phase & kPhaseUnitary; }
+
+enum PhaseShape { PH_OFF, PH_BIT, PH_PARITY, PH_OTHER };
+PhaseShape phase_shape(const StageOp &so, int gid) {
     const bool two = so.kind == SK_DIAG2;
     const bool in0 = so.dsrc[0] == 0, in1 = two && so.dsrc[1] == 0;
-    if (so.rctrl) return DS_OTHER;
-    if (!in0 && !in1) return DS_OFF;
-    if (!two) return DS_REG1;
-    if (in0 != in1) return DS_REGOFF;
-    return DS_OTHER;
+    if (so.rctrl) return PH_OTHER;
+    if (gid == GID_GP || (!in0 && !in1)) return PH_OFF;
+    if (two && gid != GID_RZZ) return PH_OTHER;
+    return in0 && in1 ? PH_PARITY : PH_BIT;
 }
-int diag_reg_bit(const StageOp &so) { return so.dsrc[0] == 0 ? so.dval[0] : so.dval[1]; }
+int phase_bit(const StageOp &so) { return so.dsrc[0] == 0 ? so.dval[0] : so.dval[1]; }
 
-// Per-thread factors of a run: sc (scalar) and f0_P / f1_P (pairs); `conj` for U^dag.
-RunPlan emit_run_factors(std::ostringstream &o, const std::vector<const StageOp *> &run, bool conj) {
-    RunPlan plan;
-    const std::string one = "cval<V>(1, 0)";
+void emit_phase_run(std::ostringstream &o, const std::vector<const StageOp *> &run, const std::vector<int> &gids, int RB,
+                    Rows *rows, StageCtx &ctx) {
+    const bool adj = rows != nullptr;
+    const int id = ctx.id++;
+    const std::string u = "_" + std::to_string(id);
     auto ent = [&](int M, const std::string &idx) {
         const std::string e = "mt[" + std::to_string(M) + " + " + idx + "]";
-        return conj ? "cconj(" + e + ")" : e;
+        return adj ? "cconj(" + e + ")" : e;
     };
-    o << "      V sc = cval<V>(1, 0);\n";
-    for (int P = 0; P < kMaxRegBits; ++P) {
-        bool used = false;
-        for (const StageOp *so : run)
-            if ((diag_shape(*so) == DS_REG1 || diag_shape(*so) == DS_REGOFF) && diag_reg_bit(*so) == P) used = true;
-        if (used) {
-            plan.bits.push_back(P);
-            o << "      V f0_" << P << " = cval<V>(1, 0), f1_" << P << " = cval<V>(1, 0);\n";
-        }
-    }
-    for (const StageOp *sp : run) {
-        const StageOp &so = *sp;
-        const std::string on = on_expr(so);
-        auto sel = [&](const std::string &v) { return on.empty() ? v : "((" + on + ") ? " + v + " : " + one + ")"; };
-        const DiagShape sh = diag_shape(so);
-        const int M = so.moff;
-        if (sh == DS_OFF) {
-            const bool two = so.kind == SK_DIAG2;
-            o << "      { const int r = " << off_bit_expr(so.dsrc[0], so.dval[0]) << " | ("
-              << off_bit_expr(two ? so.dsrc[1] : 3, so.dval[1]) << " << 1); sc = cmul(sc, " << sel(ent(M, "r")) << "); }\n";
-        } else if (sh == DS_REG1) {
-            const int P = so.dval[0];
-            o << "      f0_" << P << " = cmul(f0_" << P << ", " << sel(ent(M, "0")) << "); f1_" << P << " = cmul(f1_" << P
-              << ", " << sel(ent(M, "1")) << ");\n";
-        } else if (sh == DS_REGOFF) {
-            const int k = so.dsrc[0] == 0 ? 0 : 1;
-            const int P = so.dval[k];
-            o << "      { const int b = " << off_bit_expr(so.dsrc[1 - k], so.dval[1 - k]) << ";\n";
-            if (k == 0) o << "        const int i0 = b << 1, i1 = 1 | (b << 1);\n";
-            else o << "        const int i0 = b, i1 = 2 | b;\n";
-            o << "        f0_" << P << " = cmul(f0_" << P << ", " << sel(ent(M, "i0")) << "); f1_" << P << " = cmul(f1_" << P
-              << ", " << sel(ent(M, "i1")) << "); }\n";
-        }
-    }
-    // table over the factor bits
-    const int nb = int(plan.bits.size());
-    o << "      V T[" << (1 << nb) << "];\n      T[0] = sc;\n";
-    for (int k = 0; k < nb; ++k) {
-        const int P = plan.bits[k];
-        for (int idx = 0; idx < (1 << k); ++idx) {
-            o << "      T[" << (idx | (1 << k)) << "] = cmul(T[" << idx << "], f1_" << P << "); T[" << idx << "] = cmul(T["
-              << idx << "], f0_" << P << ");\n";
-        }
-    }
-    return plan;
-}
+    auto grads = [](const StageOp &so) { return so.n_angles ? so.grad_mask : 0; };
+    // index of a two-target entry whose register target is 0 / 1, the other target's bit in b
+    auto pair_index = [&](const StageOp &so) {
+        const int k = so.dsrc[0] == 0 ? 0 : 1;
+        const std::string b = "(" + off_bit_expr(so.dsrc[1 - k], so.dval[1 - k]) + ")";
+        return k == 0 ? std::make_pair(b + " * 2", "1 + " + b + " * 2") : std::make_pair(b, b + " + 2");
+    };
+    auto off_index = [&](const StageOp &so, int gid) {
+        if (gid == GID_GP) return std::string("0");
+        return "(" + off_bit_expr(so.dsrc[0], so.dval[0]) + " | (" +
+               off_bit_expr(so.kind == SK_DIAG2 ? so.dsrc[1] : 3, so.dval[1]) + " << 1))";
+    };
+    o << "    // " << run.size() << " diagonal gates\n";
 
-// The factor of amplitude j: table entry times the per-amplitude factors of the run's other gates.
-std::string run_factor_expr(std::ostringstream &o, const RunPlan &plan, const std::vector<const StageOp *> &run, int j,
-                            bool conj) {
-    int idx = 0;
-    for (size_t k = 0; k < plan.bits.size(); ++k)
-        if (j >> plan.bits[k] & 1) idx |= 1 << k;
-    std::string d = "T[" + std::to_string(idx) + "]";
-    const std::string one = "cval<V>(1, 0)";
-    for (const StageOp *sp : run) {
-        const StageOp &so = *sp;
-        const DiagShape sh = diag_shape(so);
-        if (sh != DS_OTHER) continue;
-        if ((uint32_t(j) & so.rctrl) != so.rctrl) continue;   // register controls not satisfied: identity
-        const std::string on = on_expr(so);
-        // entry index from the targets' bits (register bits are literals here)
-        std::string r;
-        auto bit = [&](int k) -> std::string {
-            if (so.dsrc[k] == 0) return std::to_string((j >> so.dval[k]) & 1);
-            return "(" + off_bit_expr(so.dsrc[k], so.dval[k]) + ")";
+    if (adj) {
+        // class sums of p_j = Im(conj(lambda_j) psi_j) by the register bits that the gradients depend on
+        std::vector<int> gb;
+        auto need = [&](int P) {
+            if (std::find(gb.begin(), gb.end(), P) == gb.end()) gb.push_back(P);
         };
-        if (so.kind == SK_DIAG1) r = bit(0);
-        else r = bit(0) + " | (" + bit(1) + " << 1)";
-        std::string e = "mt[" + std::to_string(so.moff) + " + (" + r + ")]";
-        if (conj) e = "cconj(" + e + ")";
-        if (!on.empty()) e = "((" + on + ") ? " + e + " : " + one + ")";
-        d = "cmul(" + d + ", " + e + ")";
-    }
-    (void)o;
-    return d;
-}
-
-void emit_forward_run(std::ostringstream &o, const std::vector<const StageOp *> &run, int RB) {
-    o << "    {   // run of " << run.size() << " diagonal gates\n";
-    const RunPlan plan = emit_run_factors(o, run, false);
-    for (int j = 0; j < (1 << RB); ++j)
-        o << "      v[" << j << "] = cmul(v[" << j << "], " << run_factor_expr(o, plan, run, j, false) << ");\n";
-    o << "    }\n";
-}
-
-void emit_backward_run(std::ostringstream &o, const std::vector<const StageOp *> &run, const std::vector<int> &gids,
-                       int RB, int NH) {
-    o << "    {   // run of " << run.size() << " diagonal gates\n";
-    // gradient sums of p_j = Im(conj(lambda_j) psi_j): all, per register bit, per special gate
-    bool any_grad = false;
-    std::vector<int> need_bits;
-    for (size_t k = 0; k < run.size(); ++k) {
-        const StageOp &so = *run[k];
-        const int G = so.n_angles ? so.grad_mask : 0;
-        if (!G) continue;
-        any_grad = true;
-        const DiagShape sh = diag_shape(so);
-        if (sh == DS_REG1 || sh == DS_REGOFF) {
-            const int P = diag_reg_bit(so);
-            if (std::find(need_bits.begin(), need_bits.end(), P) == need_bits.end()) need_bits.push_back(P);
-        }
-    }
-    if (any_grad) {
-        o << "      R S[NH] = {};\n";
-        for (int P : need_bits) o << "      R SB" << P << "[NH] = {};\n";
+        bool any = false, need_s = false;
         for (size_t k = 0; k < run.size(); ++k) {
             const StageOp &so = *run[k];
-            if ((so.n_angles ? so.grad_mask : 0) && diag_shape(so) == DS_OTHER)
-                o << "      R SX" << k << "[4][NH] = {};\n";
+            if (!grads(so)) continue;
+            any = true;
+            const PhaseShape sh = phase_shape(so, gids[k]);
+            if (sh != PH_OTHER) need_s = true;
+            if (sh == PH_BIT) need(phase_bit(so));
+            if (sh == PH_PARITY || sh == PH_OTHER)
+                for (int t = 0; t < (so.kind == SK_DIAG2 ? 2 : 1); ++t)
+                    if (so.dsrc[t] == 0) need(so.dval[t]);
+            for (int P = 0; P < RB; ++P)
+                if (so.rctrl >> P & 1) need(P);
         }
-        for (int j = 0; j < (1 << RB); ++j) {
-            o << "      for (int h = 0; h < NH; ++h) {\n        const R pj = fma(l[h][" << j << "].x, v[" << j << "].y, -l[h]["
-              << j << "].y * v[" << j << "].x);\n        S[h] += pj;";
-            for (int P : need_bits)
-                if (j >> P & 1) o << " SB" << P << "[h] += pj;";
+        if (any) {
+            const int ng = int(gb.size()), nc = 1 << ng;
+            const bool all = need_s && !ctx.S;
+            auto cls_of = [&](int j) {
+                int c = 0;
+                for (int k = 0; k < ng; ++k)
+                    if (j >> gb[size_t(k)] & 1) c |= 1 << k;
+                return c;
+            };
+            o << "    R C" << u << "[" << nc << "][NH] = {};\n    for (int h = 0; h < NH; ++h) {\n";
+            for (int j = 0; j < (1 << RB); ++j) {
+                const int c = cls_of(j);
+                if (c == 0 && !all) continue;
+                o << "     C" << u << "[" << c << "][h] = im_acc(l[h][" << j << "], v[" << j << "], C" << u << "[" << c << "][h]);\n";
+            }
+            if (all) {
+                o << "     S[h] = C" << u << "[0][h]";
+                for (int c = 1; c < nc; ++c) o << " + C" << u << "[" << c << "][h]";
+                o << ";\n";
+                ctx.S = true;
+            }
+            o << "    }\n";
+            auto sum_of = [&](const std::function<bool(int)> &in) {   // classes (bits in gb order) that `in` takes
+                std::string e;
+                for (int c = 0; c < nc; ++c)
+                    if (in(c)) e += (e.empty() ? "C" : " + C") + u + "[" + std::to_string(c) + "][h]";
+                return e.empty() ? std::string("R(0)") : "(" + e + ")";
+            };
+            auto pos = [&](int P) { return int(std::find(gb.begin(), gb.end(), P) - gb.begin()); };
             for (size_t k = 0; k < run.size(); ++k) {
                 const StageOp &so = *run[k];
-                if (!((so.n_angles ? so.grad_mask : 0) && diag_shape(so) == DS_OTHER)) continue;
-                if ((uint32_t(j) & so.rctrl) != so.rctrl) continue;
-                // class of j by the gate's register targets (off-register target bits enter the weight)
-                int cls = 0;
-                if (so.dsrc[0] == 0) cls |= (j >> so.dval[0]) & 1;
-                if (so.kind == SK_DIAG2 && so.dsrc[1] == 0) cls |= ((j >> so.dval[1]) & 1) << 1;
-                o << " SX" << k << "[" << cls << "][h] += pj;";
-            }
-            o << "\n      }\n";
-        }
-        for (size_t k = 0; k < run.size(); ++k) {
-            const StageOp &so = *run[k];
-            const int G = so.n_angles ? so.grad_mask : 0;
-            if (!G) continue;
-            const std::vector<double> pw = phase_weights(gids[k]);
-            const std::string on = on_expr(so);
-            auto onw = [&](const std::string &w) { return on.empty() ? w : "((" + on + ") ? " + w + " : R(0))"; };
-            auto wsel4 = [&](const std::string &r) {
-                return pw.size() > 2 ? "(" + r + " == 0 ? " + lit(pw[0]) + " : " + r + " == 1 ? " + lit(pw[1]) + " : " + r +
-                                           " == 2 ? " + lit(pw[2]) + " : " + lit(pw[3]) + ")"
-                                     : "(" + r + " ? " + lit(pw[1]) + " : " + lit(pw[0]) + ")";
-            };
-            o << "      {\n        R acc[3][NH];\n";
-            const DiagShape sh = diag_shape(so);
-            if (sh == DS_OFF) {
-                const bool two = so.kind == SK_DIAG2;
-                o << "        const int r = " << off_bit_expr(so.dsrc[0], so.dval[0]) << " | ("
-                  << off_bit_expr(two ? so.dsrc[1] : 3, so.dval[1]) << " << 1);\n";
-                o << "        for (int h = 0; h < NH; ++h) acc[0][h] = " << onw(wsel4("r")) << " * S[h];\n";
-            } else if (sh == DS_REG1) {
-                const int P = so.dval[0];
-                o << "        for (int h = 0; h < NH; ++h) acc[0][h] = " << onw(lit(pw[0])) << " * (S[h] - SB" << P << "[h]) + "
-                  << onw(lit(pw[1])) << " * SB" << P << "[h];\n";
-            } else if (sh == DS_REGOFF) {
-                const int kk = so.dsrc[0] == 0 ? 0 : 1;
-                const int P = so.dval[kk];
-                o << "        const int b = " << off_bit_expr(so.dsrc[1 - kk], so.dval[1 - kk]) << ";\n";
-                const std::string w_lo = kk == 0 ? "(b ? " + lit(pw[2]) + " : " + lit(pw[0]) + ")" : "(b ? " + lit(pw[1]) + " : " + lit(pw[0]) + ")";
-                const std::string w_hi = kk == 0 ? "(b ? " + lit(pw[3]) + " : " + lit(pw[1]) + ")" : "(b ? " + lit(pw[3]) + " : " + lit(pw[2]) + ")";
-                o << "        for (int h = 0; h < NH; ++h) acc[0][h] = " << onw(w_lo) << " * (S[h] - SB" << P << "[h]) + "
-                  << onw(w_hi) << " * SB" << P << "[h];\n";
-            } else {
-                // class c of SX: register target bits; off-register target bits pick the weight per thread
-                o << "        for (int h = 0; h < NH; ++h) acc[0][h] = R(0);\n";
-                for (int cls = 0; cls < 4; ++cls) {
-                    std::string r0 = so.dsrc[0] == 0 ? std::to_string(cls & 1) : "(" + off_bit_expr(so.dsrc[0], so.dval[0]) + ")";
-                    std::string r1 = "0";
-                    if (so.kind == SK_DIAG2)
-                        r1 = so.dsrc[1] == 0 ? std::to_string((cls >> 1) & 1) : "(" + off_bit_expr(so.dsrc[1], so.dval[1]) + ")";
-                    if (so.dsrc[0] != 0 && (cls & 1)) continue;
-                    if ((so.kind != SK_DIAG2 || so.dsrc[1] != 0) && (cls & 2)) continue;
-                    o << "        { const int r = " << r0 << " | (" << r1 << " << 1);\n"
-                      << "          for (int h = 0; h < NH; ++h) acc[0][h] += " << onw(wsel4("r")) << " * SX" << k << "[" << cls
-                      << "][h]; }\n";
+                if (!grads(so) || so.lslot < 0) continue;
+                const std::vector<double> pw = phase_weights(gids[k]);
+                const std::string on = on_expr(so);
+                auto wsel = [&](const std::string &r) {
+                    return pw.size() > 2 ? "(" + r + " == 0 ? " + lit(pw[0]) + " : " + r + " == 1 ? " + lit(pw[1]) + " : " + r +
+                                               " == 2 ? " + lit(pw[2]) + " : " + lit(pw[3]) + ")"
+                                         : "(" + r + " ? " + lit(pw[1]) + " : " + lit(pw[0]) + ")";
+                };
+                const PhaseShape sh = phase_shape(so, gids[k]);
+                std::string g;
+                if (sh == PH_OFF) {
+                    g = wsel(off_index(so, gids[k])) + " * S[h]";
+                } else if (sh == PH_BIT) {
+                    const int P = pos(phase_bit(so));
+                    const std::string sb = sum_of([&](int c) { return c >> P & 1; });
+                    if (so.kind == SK_DIAG1) {
+                        g = lit(pw[0]) + " * S[h] + " + lit(pw[1] - pw[0]) + " * " + sb;
+                    } else {
+                        const auto ix = pair_index(so);
+                        g = wsel("(" + ix.first + ")") + " * S[h] + (" + wsel("(" + ix.second + ")") + " - " + wsel("(" + ix.first + ")") +
+                            ") * " + sb;
+                    }
+                } else if (sh == PH_PARITY) {
+                    const int P = pos(so.dval[0]), Q = pos(so.dval[1]);
+                    g = lit(pw[0]) + " * S[h] + " + lit(pw[1] - pw[0]) + " * " +
+                        sum_of([&](int c) { return (c >> P ^ c >> Q) & 1; });
+                } else {
+                    // classes with the register controls set, by the register targets' bits
+                    for (int cls = 0; cls < 4; ++cls) {
+                        std::string r[2];
+                        bool skip = false;
+                        for (int t = 0; t < 2; ++t) {
+                            const bool there = t == 0 || so.kind == SK_DIAG2;
+                            if (there && so.dsrc[t] == 0) r[t] = std::to_string(cls >> t & 1);
+                            else if (cls >> t & 1) skip = true;
+                            else r[t] = there ? "(" + off_bit_expr(so.dsrc[t], so.dval[t]) + ")" : "0";
+                        }
+                        if (skip) continue;
+                        const std::string in = sum_of([&](int c) {
+                            for (int P = 0; P < RB; ++P)
+                                if ((so.rctrl >> P & 1) && !(c >> pos(P) & 1)) return false;
+                            for (int t = 0; t < (so.kind == SK_DIAG2 ? 2 : 1); ++t)
+                                if (so.dsrc[t] == 0 && (c >> pos(so.dval[t]) & 1) != (cls >> t & 1)) return false;
+                            return true;
+                        });
+                        g += (g.empty() ? "" : " + ") + wsel("(" + r[0] + " | (" + r[1] + " << 1))") + " * " + in;
+                    }
+                }
+                for (int h = 0; h < rows->NH; ++h) {
+                    o << "    {\n     constexpr int h = " << h << ";\n     const R g = "
+                      << (on.empty() ? g : "(" + on + ") ? " + g + " : R(0)") << ";\n";
+                    rows->put(o, "g", so.lslot, h);
+                    o << "    }\n";
                 }
             }
-            if (so.lslot >= 0)
-                o << "        for (int h = 0; h < NH; ++h) {\n          const double x = double(warp_sum_acc(acc[0][h]));\n"
-                  << "          if (lane == 0) wacc[(warp * NLS + " << so.lslot << ") * NH + h] += x;\n        }\n";
-            o << "      }\n";
         }
     }
-    const RunPlan plan = emit_run_factors(o, run, true);
-    for (int j = 0; j < (1 << RB); ++j) {
-        o << "      { const V d = " << run_factor_expr(o, plan, run, j, true) << "; v[" << j << "] = cmul(v[" << j
-          << "], d); for (int h = 0; h < NH; ++h) l[h][" << j << "] = cmul(l[h][" << j << "], d); }\n";
+
+    // the factor table over the register bits that the gates depend on
+    std::vector<int> tb;
+    auto use = [&](int P) {
+        if (std::find(tb.begin(), tb.end(), P) == tb.end()) tb.push_back(P);
+    };
+    for (size_t k = 0; k < run.size(); ++k) {
+        const StageOp &so = *run[k];
+        if (phase_shape(so, gids[k]) == PH_OFF) continue;
+        for (int t = 0; t < (so.kind == SK_DIAG2 ? 2 : 1); ++t)
+            if (so.dsrc[t] == 0) use(so.dval[t]);
+        for (int P = 0; P < RB; ++P)
+            if (so.rctrl >> P & 1) use(P);
     }
+    std::sort(tb.begin(), tb.end());
+    const int nt = 1 << tb.size();
+    std::vector<std::string> T(static_cast<size_t>(nt));   // "" is 1
+    int n_tmp = 0;
+    auto times = [&](std::string &t, const std::string &f) {
+        if (t.empty()) {
+            t = f;
+            return;
+        }
+        const std::string name = "t" + u + "_" + std::to_string(n_tmp++);
+        o << "    const V " << name << " = cmul(" << t << ", " << f << ");\n";
+        t = name;
+    };
+    auto idx_bit = [&](int idx, int P) { return (idx >> (std::find(tb.begin(), tb.end(), P) - tb.begin())) & 1; };
+    auto scale_by = [&](const std::string &f) {
+        o << "    sc = " << (ctx.sc ? "cmul(sc, " + f + ")" : f) << ";\n";
+        ctx.sc = true;
+    };
+    std::map<int, std::string> ratio;   // register bit -> product of its gates' ratios
+    for (size_t k = 0; k < run.size(); ++k) {
+        const StageOp &so = *run[k];
+        const std::string on = on_expr(so);
+        auto sel = [&](const std::string &f) { return on.empty() ? f : "((" + on + ") ? " + f + " : cval<V>(1, 0))"; };
+        const PhaseShape sh = phase_shape(so, gids[k]);
+        const bool uniform = (so.phase & kPhaseKind) == kPhaseUniform;   // d0 waits for the end of the pass, the table holds r
+        if (sh == PH_OFF && !uniform) scale_by(sel(ent(so.moff, off_index(so, gids[k]))));
+        if (sh != PH_BIT) continue;
+        const std::string r = "r" + u + "_" + std::to_string(k);
+        if (uniform) {
+            o << "    const V " << r << " = " << ent(so.moff, "1") << ";\n";
+        } else if (so.kind == SK_DIAG1) {
+            o << "    const V " << r << " = " << sel(ent(so.moff, "1")) << ";\n";
+            scale_by(sel(ent(so.moff, "0")));
+        } else {   // entries (a, b, b, a), b / a at 1: the other target's bit swaps a and b
+            const std::string b = "(" + off_bit_expr(so.dsrc[so.dsrc[0] == 0 ? 1 : 0], so.dval[so.dsrc[0] == 0 ? 1 : 0]) + ")";
+            o << "    const V " << r << "a = " << ent(so.moff, "1") << ", " << r << " = "
+              << sel("(" + b + " ? cconj(" + r + "a) : " + r + "a)") << ";\n";
+            scale_by(sel("(" + b + " ? " + ent(so.moff, "2") + " : " + ent(so.moff, "0") + ")"));
+        }
+        times(ratio[phase_bit(so)], r);
+    }
+    // products over the bits' ratios, lowest bit first
+    for (int idx = 1; idx < nt; ++idx) {
+        int top = -1;
+        for (size_t k = 0; k < tb.size(); ++k)
+            if ((idx >> k & 1) && ratio.count(tb[k])) top = int(k);
+        if (top < 0) continue;
+        T[size_t(idx)] = T[size_t(idx & ~(1 << top))];
+        // (without the bits above `top`, which carry no ratio, the entry is already there)
+        const int core = idx & ((2 << top) - 1);
+        if (core != idx) T[size_t(idx)] = T[size_t(core)];
+        else times(T[size_t(idx)], ratio[tb[size_t(top)]]);
+    }
+    for (size_t k = 0; k < run.size(); ++k) {
+        const StageOp &so = *run[k];
+        const std::string on = on_expr(so);
+        auto sel = [&](const std::string &f) { return on.empty() ? f : "((" + on + ") ? " + f + " : cval<V>(1, 0))"; };
+        const PhaseShape sh = phase_shape(so, gids[k]);
+        if (sh == PH_PARITY) {
+            const bool uniform = (so.phase & kPhaseKind) == kPhaseUniform;
+            const std::string r = "r" + u + "_" + std::to_string(k);
+            if (uniform) {
+                o << "    const V " << r << " = " << ent(so.moff, "1") << ";\n";
+            } else {
+                o << "    const V " << r << " = " << sel(ent(so.moff, "1")) << ";\n";
+                scale_by(sel(ent(so.moff, "0")));
+            }
+            for (int idx = 0; idx < nt; ++idx)
+                if (idx_bit(idx, so.dval[0]) ^ idx_bit(idx, so.dval[1])) times(T[size_t(idx)], r);
+        } else if (sh == PH_OTHER) {
+            for (int idx = 0; idx < nt; ++idx) {
+                bool set = true;
+                for (int P = 0; P < RB; ++P)
+                    if ((so.rctrl >> P & 1) && !idx_bit(idx, P)) set = false;
+                if (!set) continue;
+                std::string r;
+                for (int t = 0; t < (so.kind == SK_DIAG2 ? 2 : 1); ++t) {
+                    const std::string bit = so.dsrc[t] == 0 ? std::to_string(idx_bit(idx, so.dval[t]))
+                                                            : "(" + off_bit_expr(so.dsrc[t], so.dval[t]) + ")";
+                    r += t == 0 ? bit : " + 2 * " + bit;
+                }
+                times(T[size_t(idx)], sel(ent(so.moff, "(" + r + ")")));
+            }
+        }
+    }
+    for (int idx = 0; idx < nt; ++idx) {
+        if (T[size_t(idx)].empty()) continue;
+        o << "    {\n     const V d = " << T[size_t(idx)] << ";\n";
+        for (int j = 0; j < (1 << RB); ++j) {
+            bool in = true;
+            for (size_t k = 0; k < tb.size(); ++k) in = in && ((j >> tb[k] & 1) == (idx >> k & 1));
+            if (!in) continue;
+            o << "     v[" << j << "] = cmul(v[" << j << "], d);";
+            if (adj) o << " for (int h = 0; h < NH; ++h) l[h][" << j << "] = cmul(l[h][" << j << "], d);";
+            o << "\n";
+        }
+        o << "    }\n";
+    }
+}
+
+// The factors that a stage's diagonal gates left for its end (and, in the last stage of a pass, the pass's).
+void emit_stage_phase(std::ostringstream &o, int RB, bool adj, const StageCtx &ctx, bool last, bool pass_phase) {
+    if (!ctx.sc && !pass_phase) return;
+    const std::string ph = adj ? "cconj(*ph)" : "*ph";
+    o << "    {\n     const V d = " << (ctx.sc ? (pass_phase ? "cmul(sc, " + ph + ")" : "sc") : ph) << ";\n";
+    if (adj && last) o << "     if (a.psi_dst) {\n";   // psi leaves the last stage only where it is stored
+    for (int j = 0; j < (1 << RB); ++j) o << "     v[" << j << "] = cmul(v[" << j << "], d);\n";
+    if (adj && last) o << "     }\n";
+    if (adj)
+        for (int j = 0; j < (1 << RB); ++j)
+            o << "     for (int h = 0; h < NH; ++h) l[h][" << j << "] = cmul(l[h][" << j << "], d);\n";
     o << "    }\n";
 }
 
@@ -734,9 +802,12 @@ void emit_relayout(std::ostringstream &o, const PassPlan &pl, int K, int TB, int
 // of NB >= G tile buffers and take its tiles in turn (tile i goes to group i mod G and buffer
 // i mod NB); each group has its own matrix table (and, in the adjoint, gradient slots).  There is
 // no producer warp: a group stores its own tiles and refills their buffers, so a block of 16
-// warps keeps 128 registers per thread.  Defaults (measured on the 26-qubit HEA gradient): two
-// groups and three buffers for both kernels (forward 76 ms per step against 87 with one group of
-// two buffers, 81 with four groups; adjoint 201 ms against 219 with two buffers).  MQB_PIPE_{FWD,BWD}_{GROUPS,BUFFERS} override them (tuning).
+// warps keeps 128 registers per thread.  Defaults, measured on gradients of the 26-qubit, 12-layer ansatz (batch 2),
+// the 20-qubit classifier (64 samples) and QAOA on 26 vertices: the adjoint takes two groups and three buffers; the
+// complex64 forward pass, with 16 amplitudes per thread, one group and two buffers, so that three blocks share
+// an SM (13.4, 5.4 and 7.8 ms; two groups and three buffers 14.2, 5.2 and 8.3; one group and three buffers
+// 15.1, 5.4 and 8.0); complex128, whose tiles leave room for one block, two groups and three buffers.
+// MQB_PIPE_{FWD,BWD}_{GROUPS,BUFFERS} override them (tuning).
 int env_int(const char *name, int dflt, int lo, int hi) {
     const char *e = std::getenv(name);
     return e ? std::max(lo, std::min(hi, std::atoi(e))) : dflt;
@@ -744,17 +815,19 @@ int env_int(const char *name, int dflt, int lo, int hi) {
 
 int max_groups(int nt) { return std::max(1, std::min(15, 1024 / nt)); }
 
-int fwd_groups(const Pass &p) {
+int fwd_groups(const Pass &p, int precision) {
     const int nt = 1 << (p.K - p.f_reg_bits);
-    return std::min(max_groups(nt), env_int("MQB_PIPE_FWD_GROUPS", 2, 1, 15));
+    return std::min(max_groups(nt), env_int("MQB_PIPE_FWD_GROUPS", precision == MQB_PREC_C64 ? 1 : 2, 1, 15));
 }
 
-int fwd_buffers(const Pass &p) { return std::max(fwd_groups(p), env_int("MQB_PIPE_FWD_BUFFERS", 3, 1, 8)); }
+int fwd_buffers(const Pass &p, int precision) {
+    return std::max(fwd_groups(p, precision), env_int("MQB_PIPE_FWD_BUFFERS", precision == MQB_PREC_C64 ? 2 : 3, 1, 8));
+}
 
 size_t fwd_smem(const Pass &p, int precision) {
     const size_t eb = elem_bytes(precision);
-    return size_t(fwd_buffers(p)) * ((size_t(1) << p.K) * eb) +
-           size_t(fwd_groups(p)) * a16(size_t(p.f_mtab_entries) * eb) + 8 * 16;
+    return size_t(fwd_buffers(p, precision)) * ((size_t(1) << p.K) * eb) +
+           size_t(fwd_groups(p, precision)) * a16(size_t(p.f_mtab_entries) * eb) + 8 * 16 + 16 * size_t(eb);
 }
 
 int bwd_groups(const Pass &p) {
@@ -766,8 +839,9 @@ size_t bwd_fixed_smem(const Pass &p, int precision, int n_hams) {
     const size_t eb = elem_bytes(precision);
     const int nw = (1 << (p.K - p.reg_bits)) / 32;
     return size_t(bwd_groups(p)) *
-               (a16(size_t(p.mtab_entries) * eb) + a16(size_t(nw) * std::max(1, p.n_slots) * n_hams * sizeof(double))) +
-           8 * 16;
+               (a16(size_t(p.mtab_entries) * eb) + a16(size_t(nw) * std::max(1, p.n_slots) * n_hams * sizeof(double)) +
+                size_t(nw) * 512) +
+           8 * 16 + 16 * size_t(eb);
 }
 
 // Buffers of the adjoint ring: G + 1 where they fit in 227 KB, else as many as fit (at least G).
@@ -836,8 +910,9 @@ void emit_stage_store(std::ostringstream &o, const PassPlan &pl, const StageDesc
     o << "   }\n";
 }
 
-// The tile ring of a kernel, by its consumer groups (no producer warp).  Tile k of this block (its
-// tiles are blockIdx.x + k gridDim.x) goes to group k mod G and buffer k mod NB; the buffer is
+// The tile ring of a kernel, by its consumer groups (no producer warp).  A block has a contiguous range of
+// the tiles, so that it meets few samples: each new one costs a matrix table and a flush of the gradients (20 qubits,
+// 64 samples: a block met a new sample every 3.5 tiles when it took every 148th).  Tile k of the block goes to group k mod G and buffer k mod NB; the buffer is
 // handed over through its `full` mbarrier, with the TMA's transaction bytes, or (forward passes that
 // start from |0...0> and load nothing) with a plain arrival.  Thread 0 of block issues the first
 // NB tiles; after that the group that finished tile k stores it (thread 0 of the group, after a
@@ -852,13 +927,14 @@ void emit_stage_store(std::ostringstream &o, const PassPlan &pl, const StageDesc
 void emit_ring_prologue(std::ostringstream &o, const std::string &issue_body, bool zero_opt) {
     o << "  const int grp = int(threadIdx.x) / NT, BAR = 1 + grp;\n"
       << "  const unsigned tid = threadIdx.x % NT;\n"
-      << "  const long long first = blockIdx.x, cnt = first < total ? (total - 1 - first) / gridDim.x + 1 : 0;\n"
+      << "  const long long share = total / gridDim.x, more = total % gridDim.x, bi = blockIdx.x;\n"
+      << "  const long long first = bi * share + (bi < more ? bi : more), cnt = share + (bi < more);\n"
       << "  const int n = a.g.n;\n"
       << "  long long mine[NB];\n"
       << "  for (int k = 0; k < NB; ++k) mine[k] = -1;\n"
       << "  auto issue = [&](long long k) {\n"
       << "   const int sb = int(k % NB);\n"
-      << "   const long long w = first + k * gridDim.x, b = w >> a.g.n_out;\n"
+      << "   const long long w = first + k, b = w >> a.g.n_out;\n"
       << "   const tile::u64 tb = tile::tile_base(a.g, tile::u64(w) & tile::u64(n_tiles - 1));\n"
       << "   unsigned char *buf = smem + sb * BUFB;\n"
       << "   mine[sb] = k;\n"
@@ -902,15 +978,18 @@ void emit_ring_exit(std::ostringstream &o) {
       << "   pipe::bulk_wait_all();\n  }\n";
 }
 
-std::string forward_source(const Schedule &s, const Pass &p, int precision) {
+std::string forward_source(const Schedule &s, const Pass &p, int precision, const std::vector<DevOp> &ops) {
     const int RB = p.f_reg_bits, K = p.K, TB = K - RB;
     const PassPlan pl = pass_plan(p.qbits, precision);
-    const int NB = fwd_buffers(p), G = fwd_groups(p);
+    const int NB = fwd_buffers(p, precision), G = fwd_groups(p, precision);
     std::vector<const StageDesc *> ex;
     for (int si = 0; si < p.f_n_stages; ++si) ex.push_back(&s.f_stages[p.f_stage_begin + si]);
     const LayPlan lp = plan_layouts(pl, ex, TB);
-    // blocks per SM that the shared-memory ring allows: the register budget is sized for them
-    const int min_blocks = int(std::max<size_t>(1, std::min<size_t>(3, (size_t(220) << 10) / fwd_smem(p, precision))));
+    bool pass_phase = false;
+    for (int k = 0; k < p.f_n_sops; ++k) pass_phase = pass_phase || leaves_factor(s.f_stage_ops[p.f_sop_begin + k]);
+    // blocks per SM that the shared-memory ring allows, up to 24 warps: the register budget is sized for them
+    const size_t fit = (size_t(220) << 10) / fwd_smem(p, precision), most = size_t(768) / size_t(G << TB);
+    const int min_blocks = int(std::max<size_t>(1, std::min(most, fit)));
     std::ostringstream o;
     emit_header(o, precision);
     o << "extern \"C\" __global__ void __launch_bounds__(" << G * (1 << TB) << ", " << min_blocks
@@ -923,6 +1002,7 @@ std::string forward_source(const Schedule &s, const Pass &p, int precision) {
       << "  const tile::u64 mtb = tile::align16(tile::u64(a.mtab_entries) * sizeof(V));\n"
       << "  pipe::u64 *full = reinterpret_cast<pipe::u64 *>(smem + NB * BUFB + G * mtb);\n"
       << "  volatile long long *ticket = reinterpret_cast<volatile long long *>(full + NB);\n"
+      << "  V *ph = reinterpret_cast<V *>(full + 16) + int(threadIdx.x) / NT;   // factor left for the end of the pass\n"
       << "  if (threadIdx.x == 0) {\n   for (int k = 0; k < NB; ++k) {\n    pipe::mbar_init(full + k, 1);\n    ticket[k] = -1;\n   }\n"
       << "   pipe::fence_mbar_init();\n  }\n  __syncthreads();\n"
       << "  const long long n_tiles = 1ll << a.g.n_out, total = a.batch * n_tiles;\n"
@@ -934,13 +1014,14 @@ std::string forward_source(const Schedule &s, const Pass &p, int precision) {
     o << "  V *mt = reinterpret_cast<V *>(smem + NB * BUFB + grp * mtb);\n"
       << "  long long cached_b = -1;\n"
       << "  for (long long i = grp; i < cnt; i += G) {\n"
-      << "   const long long w = first + i * gridDim.x, b = w >> a.g.n_out;\n"
+      << "   const long long w = first + i, b = w >> a.g.n_out;\n"
       << "   const tile::u64 base = tile::tile_base(a.g, tile::u64(w) & tile::u64(n_tiles - 1));\n"
       << "   const int sb = int(i % NB);\n   const unsigned par = unsigned(i / NB) & 1u;\n"
       << "   V *tl = reinterpret_cast<V *>(smem + sb * BUFB);\n"
       << "   if (b != cached_b) {\n    pipe::consumers_sync(BAR, NT);\n"
       << "    pipe::load_mtab(mt, a.mt, a.n_mt, a.mats + b * a.mats_stride, a.cpool, tid, NT);\n"
-      << "    cached_b = b;\n    pipe::consumers_sync(BAR, NT);\n   }\n";
+      << "    cached_b = b;\n    pipe::consumers_sync(BAR, NT);\n"
+      << (pass_phase ? "    pipe::pass_phase(ph, mt, a.mt, a.n_mt, tid);\n    pipe::consumers_sync(BAR, NT);\n" : "") << "   }\n";
     emit_ring_wait(o);
     if (lp.relayout_in) {
         o << "   if (!zero) {\n    V *tbase = tl;\n";
@@ -951,18 +1032,21 @@ std::string forward_source(const Schedule &s, const Pass &p, int precision) {
         const StageDesc &sd = *ex[si];
         const bool last = si + 1 == ex.size();
         emit_stage_load(o, pl, sd, RB, TB, 0, lp.in[si], si == 0);
+        StageCtx ctx;
+        o << "    V sc = cval<V>(1, 0);\n";
         for (int k = sd.op_begin; k < sd.op_end;) {
             std::vector<const StageOp *> run;
-            int e = k;
-            while (e < sd.op_end && diag_op(s.f_stage_ops[p.f_sop_begin + e])) run.push_back(&s.f_stage_ops[p.f_sop_begin + e++]);
-            if (run.size() >= 2) {
-                emit_forward_run(o, run, RB);
-                k = e;
-            } else {
-                emit_forward_op(o, s.f_stage_ops[p.f_sop_begin + k]);
-                ++k;
+            std::vector<int> gids;
+            for (; k < sd.op_end; ++k) {
+                const StageOp &so = s.f_stage_ops[p.f_sop_begin + k];
+                if (!phase_op(so, ops[so.op].gate_id, false)) break;
+                run.push_back(&so);
+                gids.push_back(ops[so.op].gate_id);
             }
+            if (!run.empty()) emit_phase_run(o, run, gids, RB, nullptr, ctx);
+            else emit_forward_op(o, s.f_stage_ops[p.f_sop_begin + k++]);
         }
+        emit_stage_phase(o, RB, false, ctx, last, last && pass_phase);
         if (last)   // the FP64 norm check of the output, when the launch asks for it
             o << "    if (a.norm) {\n     double ns = 0;\n"
               << "     for (int j = 0; j < NR; ++j) ns += double(v[j].x) * double(v[j].x) + double(v[j].y) * double(v[j].y);\n"
@@ -989,8 +1073,12 @@ std::string backward_source(const Schedule &s, const Pass &p, int precision, int
     std::vector<const StageDesc *> ex;
     for (int si = p.n_stages - 1; si >= 0; --si) ex.push_back(&s.stages[p.stage_begin + si]);
     const LayPlan lp = plan_layouts(pl, ex, TB);
+    bool pass_phase = false;
+    for (int k = 0; k < p.n_sops; ++k) pass_phase = pass_phase || leaves_factor(s.stage_ops[p.sop_begin + k]);
+    Rows rows;
+    rows.batch = row_batch(precision);
+    rows.NH = NH;
     std::ostringstream o;
-    emit_header(o, precision);
     o << "extern \"C\" __global__ void __launch_bounds__(" << G * (1 << TB) << ", 1) mqb_adj_pass(const JitBwdArgs<V> a, "
       << "const __grid_constant__ pipe::TMap m_psi, const __grid_constant__ pipe::TMap m_lam, "
       << "const __grid_constant__ pipe::TMap m_pdst) {\n"
@@ -1003,6 +1091,7 @@ std::string backward_source(const Schedule &s, const Pass &p, int precision, int
       << "  double *wacc0 = reinterpret_cast<double *>(smem + NB * BUFB + G * mtb);\n"
       << "  pipe::u64 *full = reinterpret_cast<pipe::u64 *>(wacc0 + G * WS);\n"
       << "  volatile long long *ticket = reinterpret_cast<volatile long long *>(full + NB);\n"
+      << "  V *ph = reinterpret_cast<V *>(full + 16) + int(threadIdx.x) / NT;   // factor left for the end of the pass\n"
       << "  if (threadIdx.x == 0) {\n   for (int k = 0; k < NB; ++k) {\n    pipe::mbar_init(full + k, 1);\n    ticket[k] = -1;\n   }\n"
       << "   pipe::fence_mbar_init();\n  }\n"
       << "  for (int i = int(threadIdx.x); i < G * WS; i += int(blockDim.x)) wacc0[i] = 0;\n  __syncthreads();\n"
@@ -1015,16 +1104,18 @@ std::string backward_source(const Schedule &s, const Pass &p, int precision, int
                        false);
     o << "  const int warp = int(tid) / 32, lane = int(tid) % 32;\n"
       << "  V *mt = reinterpret_cast<V *>(smem + NB * BUFB + grp * mtb);\n"
-      << "  double *wacc = wacc0 + grp * WS;\n"
+      << "  double *wacc = wacc0 + grp * WS, *wrow = wacc + warp * NLS * NH;\n"
+      << "  const unsigned scr = pipe::saddr(reinterpret_cast<V *>(full + 16) + 16) + unsigned(grp * nw + warp) * 512u;\n"
       << "  long long cached_b = -1;\n"
       << "  for (long long i = grp; i < cnt; i += G) {\n"
-      << "   const long long w = first + i * gridDim.x, b = w >> a.g.n_out;\n"
+      << "   const long long w = first + i, b = w >> a.g.n_out;\n"
       << "   const tile::u64 base = tile::tile_base(a.g, tile::u64(w) & tile::u64(n_tiles - 1));\n"
       << "   const int sb = int(i % NB);\n   const unsigned par = unsigned(i / NB) & 1u;\n"
       << "   V *psi = reinterpret_cast<V *>(smem + sb * BUFB);\n   V *lam = psi + TS;\n"
       << "   if (b != cached_b) {\n    pipe::consumers_sync(BAR, NT);\n"
       << "    pipe::load_mtab(mt, a.mt, a.n_mt, a.mats + b * a.mats_stride, a.cpool, tid, NT);\n"
-      << "    cached_b = b;\n    pipe::consumers_sync(BAR, NT);\n   }\n";
+      << "    cached_b = b;\n    pipe::consumers_sync(BAR, NT);\n"
+      << (pass_phase ? "    pipe::pass_phase(ph, mt, a.mt, a.n_mt, tid);\n    pipe::consumers_sync(BAR, NT);\n" : "") << "   }\n";
     emit_ring_wait(o);
     if (lp.relayout_in) {
         o << "   {\n    V *tbase = psi;\n";
@@ -1035,28 +1126,29 @@ std::string backward_source(const Schedule &s, const Pass &p, int precision, int
         const StageDesc &sd = *ex[si];
         const bool last = si + 1 == ex.size();
         emit_stage_load(o, pl, sd, RB, TB, NH, lp.in[si], false);
+        StageCtx ctx;
+        o << "    V sc = cval<V>(1, 0);\n    R S[NH];\n";
         for (int k = sd.op_end - 1; k >= sd.op_begin;) {
             std::vector<const StageOp *> run;
             std::vector<int> gids;
-            int e = k;
-            while (e >= sd.op_begin) {
-                const StageOp &so = s.stage_ops[p.sop_begin + e];
-                if (!run_ok_backward(so, ops[so.op].gate_id)) break;
+            for (; k >= sd.op_begin; --k) {
+                const StageOp &so = s.stage_ops[p.sop_begin + k];
+                if (!phase_op(so, ops[so.op].gate_id, true)) break;
                 run.push_back(&so);
                 gids.push_back(ops[so.op].gate_id);
-                --e;
             }
-            if (run.size() >= 2) {
-                emit_backward_run(o, run, gids, RB, NH);
-                k = e;
+            if (!run.empty()) {
+                emit_phase_run(o, run, gids, RB, &rows, ctx);
             } else {
-                const StageOp &so = s.stage_ops[p.sop_begin + k];
-                emit_backward_op(o, so, NH, ops[so.op].gate_id);
-                --k;
+                const StageOp &so = s.stage_ops[p.sop_begin + k--];
+                emit_backward_op(o, so, NH, ops[so.op].gate_id, rows);
+                ctx.S = ctx.S && keeps_sums(so);
             }
         }
+        emit_stage_phase(o, RB, true, ctx, last, last && pass_phase);
         emit_stage_store(o, pl, sd, RB, TB, NH, lp.in[si], lp.out[si], !last || lp.relayout_out);
     }
+    if (int(rows.order.size()) % rows.batch) rows.flush(o);
     if (lp.relayout_out) {
         o << "   {\n    V *tbase = psi;\n";
         emit_relayout(o, pl, K, TB, 1 + NH, false);
@@ -1067,18 +1159,23 @@ std::string backward_source(const Schedule &s, const Pass &p, int precision, int
                     "     pipe::store_tile(&m_lam, a.tg, (tile::u64(h * a.batch + b) << n) | base, buf + (1 + h) * TILEB);\n"
                     "    if (a.psi_dst) pipe::store_tile(&m_pdst, a.tg, (tile::u64(b) << n) | base, buf);\n");
     o << "   const long long nxt = i + G;\n"
-      << "   if (nxt >= cnt || ((first + nxt * gridDim.x) >> a.g.n_out) != b) {\n"
+      << "   if (nxt >= cnt || ((first + nxt) >> a.g.n_out) != b) {\n"
       << "    pipe::consumers_sync(BAR, NT);\n"
       << "    for (int s2 = int(tid); s2 < a.n_local_slots * NH; s2 += NT) {\n"
       << "     double sum = 0;\n"
       << "     for (int ww = 0; ww < nw; ++ww) {\n"
       << "      sum += wacc[ww * NLS * NH + s2];\n      wacc[ww * NLS * NH + s2] = 0;\n     }\n"
-      << "     const int ls = s2 / NH, h = s2 % NH;\n"
+      << "     const int ls = row_slot[s2] / NH, h = row_slot[s2] % NH;\n"
       << "     if (sum != 0) atomicAdd(&a.gslots[(b * a.n_slots + a.slot_map[ls]) * a.n_hams + h], sum);\n"
       << "    }\n    pipe::consumers_sync(BAR, NT);\n   }\n  }\n";
     emit_ring_exit(o);
     o << "}\n";
-    return o.str();
+    std::ostringstream head;
+    emit_header(head, precision);
+    head << "__constant__ unsigned short row_slot[" << std::max<size_t>(1, rows.order.size()) << "] = {";
+    for (size_t i = 0; i < rows.order.size(); ++i) head << (i ? ", " : "") << rows.order[i];
+    head << "};   // gradient row -> pass-local slot * NH + Hamiltonian\n";
+    return head.str() + o.str();
 }
 
 // On-disk cache of the cubins compiled here, so a new process does not compile the same pass
@@ -1100,7 +1197,7 @@ std::string compile_input(const Entry &e, const char *const *opts, int n_opts) {
     nvrtcVersion(&major, &minor);
     std::string in = "nvrtc " + std::to_string(major) + "." + std::to_string(minor) + "\n";
     for (int i = 0; i < n_opts; ++i) in += std::string(opts[i]) + "\n";
-    for (const char *h : {kJitRegmath, kJitTile, kJitAbi, kJitPipe}) in += std::string(h) + "\n";
+    for (const char *h : {kJitRegmath, kJitTile, kJitAbi, kJitPipe, kJitPhase}) in += std::string(h) + "\n";
     return in + e.src;
 }
 
@@ -1142,9 +1239,9 @@ void compile_entry(Entry &e) {
         }
     }
     nvrtcProgram prog = nullptr;
-    const char *hdrs[4] = {kJitRegmath, kJitTile, kJitAbi, kJitPipe};
-    const char *names[4] = {"regmath.cuh", "tile.cuh", "jit_abi.h", "pipe.cuh"};
-    if (nvrtcCreateProgram(&prog, e.src.c_str(), "mqb_pass.cu", 4, hdrs, names) != NVRTC_SUCCESS) {
+    const char *hdrs[5] = {kJitRegmath, kJitTile, kJitAbi, kJitPipe, kJitPhase};
+    const char *names[5] = {"regmath.cuh", "tile.cuh", "jit_abi.h", "pipe.cuh", "phasemath.cuh"};
+    if (nvrtcCreateProgram(&prog, e.src.c_str(), "mqb_pass.cu", 5, hdrs, names) != NVRTC_SUCCESS) {
         e.log = "nvrtcCreateProgram failed";
         return;
     }
@@ -1237,18 +1334,18 @@ std::vector<const void *> kernels_for(const std::vector<std::string> &srcs) {
 
 }  // namespace
 
-std::string jit_forward_source(const Schedule &s, const Pass &p, int precision) {
-    return forward_source(s, p, precision);
+std::string jit_forward_source(const Schedule &s, const Pass &p, int precision, const std::vector<DevOp> &ops) {
+    return forward_source(s, p, precision, ops);
 }
 std::string jit_backward_source(const Schedule &s, const Pass &p, int precision, int n_hams,
                                 const std::vector<DevOp> &ops) {
     return backward_source(s, p, precision, n_hams, ops);
 }
 
-std::vector<const void *> jit_forward_kernels(const Schedule &s, int precision) {
+std::vector<const void *> jit_forward_kernels(const Schedule &s, int precision, const std::vector<DevOp> &ops) {
     std::vector<std::string> srcs(s.passes.size());
     for (size_t i = 0; i < s.passes.size(); ++i)
-        if (s.passes[i].fused) srcs[i] = forward_source(s, s.passes[i], precision);
+        if (s.passes[i].fused) srcs[i] = forward_source(s, s.passes[i], precision, ops);
     return kernels_for(srcs);
 }
 
@@ -1264,7 +1361,7 @@ int jit_compile_check(const Schedule &s, int precision, int n_hams, const std::v
     std::vector<std::string> srcs;
     for (const Pass &p : s.passes) {
         if (!p.fused) continue;
-        srcs.push_back(forward_source(s, p, precision));
+        srcs.push_back(forward_source(s, p, precision, ops));
         if (n_hams > 0) srcs.push_back(backward_source(s, p, precision, n_hams, ops));
     }
     std::sort(srcs.begin(), srcs.end());
@@ -1396,7 +1493,7 @@ cudaError_t jit_launch_forward(const void *kernel, JitFwdArgs<V> a, const Pass &
     encode_map(&ms, a.src, a.g.n, a.src_batch_stride ? a.batch : 1, pl);
     encode_map(&md, a.dst, a.g.n, a.batch, pl);
     void *argv[] = {&a, &ms, &md};
-    return launch_pipe(kernel, argv, fwd_groups(p) * (1 << (p.K - p.f_reg_bits)), jit_forward_smem(p, precision), sm_count,
+    return launch_pipe(kernel, argv, fwd_groups(p, precision) * (1 << (p.K - p.f_reg_bits)), jit_forward_smem(p, precision), sm_count,
                        a.batch << a.g.n_out, st);
 }
 

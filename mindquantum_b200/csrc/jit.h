@@ -13,9 +13,9 @@
 
 namespace mqb {
 
-// Per pass of `s`: the forward kernel (nullptr for unfused passes).  Compiles what the cache
+// Per pass of `s`: the forward kernel (nullptr for unfused passes; `ops`: the program's lowered gates).  Compiles what the cache
 // lacks, in parallel; throws std::runtime_error with the compiler log on failure.
-std::vector<const void *> jit_forward_kernels(const Schedule &s, int precision);
+std::vector<const void *> jit_forward_kernels(const Schedule &s, int precision, const std::vector<DevOp> &ops);
 // Per pass of `s`: the backward kernel for n_hams lambdas (`ops`: the program's lowered gates).
 std::vector<const void *> jit_backward_kernels(const Schedule &s, int precision, int n_hams,
                                                const std::vector<DevOp> &ops);
@@ -48,7 +48,7 @@ void tile_tma_map(void *map, const void *base, int n, long long outer, const std
 int jit_compile_check(const Schedule &s, int precision, int n_hams, const std::vector<DevOp> &ops);
 
 // Sources of the kernels of one pass (for tests and inspection).
-std::string jit_forward_source(const Schedule &s, const Pass &p, int precision);
+std::string jit_forward_source(const Schedule &s, const Pass &p, int precision, const std::vector<DevOp> &ops);
 std::string jit_backward_source(const Schedule &s, const Pass &p, int precision, int n_hams,
                                 const std::vector<DevOp> &ops);
 

@@ -43,6 +43,8 @@ struct DevOp {
     uint64_t px, py, pz;         // GID_RPS masks
     int32_t pny;
     int32_t sub;                 // dense single-qubit structure: SUB_GENERIC, SUB_REAL, SUB_PERM, SUB_SWAP, SUB_RXL
+    int32_t unitary;             // 1: unitary whatever its parameters (0: a custom gate or a matrix that is not)
+    int32_t pad;
 };
 // Structure of a dense single-qubit matrix, used to pick a cheaper register kernel.
 // SUB_RXL: [[a, ib], [ib, a]] with a, b real, and so are its derivatives (RX).
@@ -118,8 +120,15 @@ struct StageOp {
     int32_t code;        // RegCode of the forward kernels
     int32_t bcode;       // code * 4 + gradient selector, for the backward kernels
     int32_t cflags;      // bit 0: octrl != 0, bit 1: tctrl != 0 (controls checked per thread)
-    int32_t pad;
+    int32_t phase;       // generated kernels: a StagePhase kind, and kPhaseUnitary
 };
+
+// StageOp::phase, for the generated kernels: a diagonal gate whose table holds the ratio of its pair, with the
+// first entry the same for every thread, so that it waits for the end of the pass (kPhaseUniform: uncontrolled,
+// on register bits, or a global phase), or not (kPhasePair); a flag of the gates known to be unitary; and from bit
+// kPhaseNormShift on, for the uncontrolled gates of a complex64 pass, the entries of M whose mean square says by
+// how much rounding took the gate away from norm one (0: not counted; kPhaseDiag: they are a diagonal's).
+enum StagePhase : int32_t { kPhaseUniform = 1, kPhasePair = 2, kPhaseKind = 3, kPhaseUnitary = 4, kPhaseDiag = 128, kPhaseNormShift = 8 };
 
 // A pass: one sweep over the state(s).
 struct Pass {
@@ -219,6 +228,11 @@ int contiguity_bits(int precision);
 int default_tile_bits(int precision, int n_states_in_tile);
 // Register bits of the fused kernels: forward passes, and backward passes with n_hams lambdas.
 int fwd_reg_bits(int precision);
+// The same for the generated forward kernels: 4 for complex64.  16 amplitudes per thread take half the code of 32,
+// which is straight-line and bound by instruction fetch as much as by arithmetic, at the price of more
+// stages: 26 qubits x 12 layers 14.1 -> 13.2 ms of forward passes (batch 2), the 20-qubit classifier 6.6 -> 5.4, QAOA
+// on 26 vertices 9.3 -> 7.8; compiling takes half the time.
+int jit_fwd_reg_bits(int precision);
 int bwd_reg_bits(int precision, int n_hams);
 
 }  // namespace mqb

@@ -9,6 +9,7 @@
 #define MQB_PIPE_CUH_
 
 #include "jit_abi.h"
+#include "phasemath.cuh"
 
 namespace mqb {
 namespace pipe {
@@ -103,7 +104,8 @@ __device__ __forceinline__ bool consumers_and(int id, int n, bool q) {
     return r != 0;
 }
 
-// The matrices of a pass's ops into shared memory, by the nt consumer threads (one warp per op).
+// The matrices of a pass's ops into shared memory, by the nt consumer threads (one warp per op), with the
+// ratios of the diagonal pairs.
 template <typename V>
 __device__ __forceinline__ void load_mtab(V *mtab, const JitMtab *mt, int n, const V *mb, const V *cpool, unsigned tid,
                                           unsigned nt) {
@@ -112,7 +114,92 @@ __device__ __forceinline__ void load_mtab(V *mtab, const JitMtab *mt, int n, con
         const JitMtab e = mt[k];
         const V *src = (e.msrc_ps ? mb : cpool) + e.msrc;
         for (int i = static_cast<int>(lane); i < e.mcount; i += 32) mtab[e.moff + i] = src[i];
+        if (e.phase & 3) {
+            __syncwarp();
+            if (lane == 0) reg::prepare_pair(mtab + e.moff);
+        }
     }
+}
+
+// The factor left for the end of a pass, made by the group's first warp after the table is complete: the product
+// of the uniform diagonal pairs' first entries, over the norms that rounding gave the uncontrolled gates.  A
+// complex64 rotation's c and s leave c^2 + s^2 off one by some 1e-8, the same for every amplitude, so over
+// hundreds of gates the state's norm drifted by 1e-6 and took the expectation and the gradients along; one
+// factor per pass takes it out.
+template <typename V>
+__device__ __forceinline__ void pass_phase(V *ph, const V *mtab, const JitMtab *mt, int n, unsigned tid) {
+    if (tid >= 32u) return;
+    double2 p = reg::cval<double2>(1, 0);
+    for (int k = static_cast<int>(tid); k < n; k += 32) {
+        const JitMtab e = mt[k];
+        const V *M = mtab + e.moff;
+        const int kind = e.phase & 3, norm = e.phase >> 8;
+        double q = 1;   // mean square of what the gate multiplies amplitudes by
+        auto sq = [&](int i) { return double(M[i].x) * double(M[i].x) + double(M[i].y) * double(M[i].y); };
+        if (kind == 1) p = reg::unit(reg::cmul(p, reg::wide(M[0])));
+        if (norm) {
+            if (kind == 1) {            // (1, r)
+                q = 0.5 * (1.0 + sq(1));
+            } else if (kind == 2) {     // d0 = M[0] or M[2], times (1, r) or (1, conj r)
+                q = 0.25 * (sq(0) + sq(2)) * (1.0 + sq(1));
+            } else {                    // 4^m entries of 2^m rows, or a diagonal of 2^m
+                q = 0;
+                for (int i = 0; i < norm; ++i) q += sq(i);
+                q /= e.phase & 128 ? norm : norm == 16 ? 4 : 2;
+            }
+            const double t = 1.5 - 0.5 * q;   // 1 / sqrt(q) for q this close to one
+            p.x *= t;
+            p.y *= t;
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        double2 q;
+        q.x = __shfl_xor_sync(0xffffffffu, p.x, o);
+        q.y = __shfl_xor_sync(0xffffffffu, p.y, o);
+        p = reg::cmul(p, q);
+    }
+    if (tid == 0u) *ph = reg::cval<V>(p.x, p.y);
+}
+
+// Gradient rows of a warp: 512 bytes of shared scratch at `scr` hold 4 rows of 32 float partials (2 of
+// double).  row_put stores this lane's partial of row k; rows_flush_as adds the n rows over the lanes (in
+// the partials' precision) and the sums to acc[0..n) in FP64.  The accesses are volatile asm without a
+// memory clobber: they keep their order among themselves, and the compiler may move the gates' own
+// shared-memory reads across them.
+__device__ __forceinline__ void row_put(unsigned scr, int k, int lane, float x) {
+    asm volatile("st.shared.f32 [%0], %1;" ::"r"(scr + unsigned(k * 32 + lane) * 4u), "f"(x));
+}
+__device__ __forceinline__ void row_put(unsigned scr, int k, int lane, double x) {
+    asm volatile("st.shared.f64 [%0], %1;" ::"r"(scr + unsigned(k * 32 + lane) * 8u), "d"(x));
+}
+__device__ __forceinline__ void rows_sum(unsigned scr, int lane, float &s, int &row, bool &first) {
+    float x, y, z, w;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x), "=f"(y), "=f"(z), "=f"(w) : "r"(scr + unsigned(lane) * 16u));
+    s = (x + y) + (z + w);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    row = lane >> 3;
+    first = (lane & 7) == 0;
+}
+__device__ __forceinline__ void rows_sum(unsigned scr, int lane, double &s, int &row, bool &first) {
+    double x, y;
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(x), "=d"(y) : "r"(scr + unsigned(lane) * 16u));
+    s = x + y;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    row = lane >> 4;
+    first = (lane & 15) == 0;
+}
+__device__ __forceinline__ void warp_order() { asm volatile("bar.warp.sync 0xffffffff;"); }
+template <typename R>
+__device__ __forceinline__ void rows_flush_as(unsigned scr, double *acc, int n, int lane) {
+    R s;
+    int row;
+    bool first;
+    warp_order();
+    rows_sum(scr, lane, s, row, first);
+    warp_order();
+    if (first && row < n) acc[row] += double(s);
 }
 
 // Make this thread's generic-proxy writes to shared memory visible to the TMA (async proxy).

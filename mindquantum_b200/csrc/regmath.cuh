@@ -521,74 +521,6 @@ __device__ __forceinline__ void jbg_rx(V (&v)[1 << RB], V (&l)[NH][1 << RB], R a
     for (int h = 0; h < NH; ++h) acc[0][h] += gs * g[h];
 }
 
-// Diagonal phase gates (RZ, RZZ, PS, GP): dU/dt = -i W U with W diagonal and real, so the
-// gradient is sum_j w_j Im(conj(l_j) x_j).  One target on register P: weights (w0, w1) by bit P;
-// c0, c1 = conj of the entries for the uncompute.
-template <typename V, int RB, int NH, int P, unsigned CM, typename R>
-__device__ __forceinline__ void jbg_diag1(V (&v)[1 << RB], V (&l)[NH][1 << RB], V c0, V c1, R w0, R w1,
-                                          R (&acc)[3][NH]) {
-    R g0[NH], g1[NH];
-#pragma unroll
-    for (int h = 0; h < NH; ++h) g0[h] = g1[h] = 0;
-#pragma unroll
-    for (int j = 0; j < (1 << RB); ++j) {
-        if (!ctl_on<CM>(j)) continue;
-        const bool hi = (j >> P) & 1;
-#pragma unroll
-        for (int h = 0; h < NH; ++h) {
-            if (hi) g1[h] = im_acc(l[h][j], v[j], g1[h]);
-            else g0[h] = im_acc(l[h][j], v[j], g0[h]);
-        }
-        v[j] = cmul(v[j], hi ? c1 : c0);
-#pragma unroll
-        for (int h = 0; h < NH; ++h) l[h][j] = cmul(l[h][j], hi ? c1 : c0);
-    }
-#pragma unroll
-    for (int h = 0; h < NH; ++h) acc[0][h] += w0 * g0[h] + w1 * g1[h];
-}
-
-// two targets on registers P (matrix bit 0) and Q (matrix bit 1): weights w[r], r = b0 | b1 << 1
-template <typename V, int RB, int NH, int P, int Q, unsigned CM, typename R>
-__device__ __forceinline__ void jbg_diag2(V (&v)[1 << RB], V (&l)[NH][1 << RB], const V (&c)[4], const R (&w)[4],
-                                          R (&acc)[3][NH]) {
-    R g[4][NH];
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int h = 0; h < NH; ++h) g[r][h] = 0;
-#pragma unroll
-    for (int j = 0; j < (1 << RB); ++j) {
-        if (!ctl_on<CM>(j)) continue;
-        const int r = ((j >> P) & 1) | (((j >> Q) & 1) << 1);
-#pragma unroll
-        for (int h = 0; h < NH; ++h) g[r][h] = im_acc(l[h][j], v[j], g[r][h]);
-        v[j] = cmul(v[j], c[r]);
-#pragma unroll
-        for (int h = 0; h < NH; ++h) l[h][j] = cmul(l[h][j], c[r]);
-    }
-#pragma unroll
-    for (int h = 0; h < NH; ++h) acc[0][h] += w[0] * g[0][h] + w[1] * g[1][h] + w[2] * g[2][h] + w[3] * g[3][h];
-}
-
-// targets off the registers: one entry c and one weight w per thread
-template <typename V, int RB, int NH, unsigned CM, typename R>
-__device__ __forceinline__ void jbg_scale(V (&v)[1 << RB], V (&l)[NH][1 << RB], V c, R w, R (&acc)[3][NH]) {
-    R g[NH];
-#pragma unroll
-    for (int h = 0; h < NH; ++h) g[h] = 0;
-#pragma unroll
-    for (int j = 0; j < (1 << RB); ++j) {
-        if (!ctl_on<CM>(j)) continue;
-#pragma unroll
-        for (int h = 0; h < NH; ++h) g[h] = im_acc(l[h][j], v[j], g[h]);
-        v[j] = cmul(v[j], c);
-#pragma unroll
-        for (int h = 0; h < NH; ++h) l[h][j] = cmul(l[h][j], c);
-    }
-#pragma unroll
-    for (int h = 0; h < NH; ++h) acc[0][h] += w * g[h];
-}
-
 // dense 4x4 from the matrix table: M = U (row-major), dM_a = M + 16 (1 + a)
 template <typename V, int RB, int NH, int P, int Q, unsigned CM, int G>
 __device__ __forceinline__ void jb_dense2(V (&v)[1 << RB], V (&l)[NH][1 << RB], const V *M,

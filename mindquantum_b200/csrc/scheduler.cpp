@@ -31,6 +31,8 @@ int fwd_reg_bits(int precision) {
     return precision == MQB_PREC_C64 ? 5 : 4;
 }
 
+int jit_fwd_reg_bits(int precision) { return precision == MQB_PREC_C64 ? std::min(4, fwd_reg_bits(precision)) : fwd_reg_bits(precision); }
+
 int bwd_reg_bits(int precision, int n_hams) {
     if (n_hams <= 1) return precision == MQB_PREC_C64 ? 4 : 3;
     return precision == MQB_PREC_C64 ? 3 : 2;
@@ -527,6 +529,17 @@ void build_stages(Schedule &s, const std::vector<DevOp> &ops, int reg_bits, int 
                     }
                 }
                 assign_codes(so);
+                if (dop.unitary) {
+                    so.phase = kPhaseUnitary;
+                    const bool reg0 = so.dsrc[0] == 0, reg1 = so.dsrc[1] == 0;
+                    const bool one = so.kind == SK_DIAG1 && reg0, zz = so.kind == SK_DIAG2 && dop.gate_id == GID_RZZ;
+                    if ((so.kind == SK_DIAG1 && dop.gate_id == GID_GP) || one || (zz && reg0 && reg1))
+                        so.phase |= dop.ctrl ? (one && !so.rctrl && dop.gate_id != GID_GP ? kPhasePair : 0) : kPhaseUniform;
+                    else if (zz && (reg0 || reg1) && !so.rctrl)
+                        so.phase |= kPhasePair;
+                    if (zz && reg0 && reg1 && dop.ctrl && !so.rctrl) so.phase |= kPhasePair;
+                    if (precision == MQB_PREC_C64 && !dop.ctrl && so.kind != SK_SWAP1) so.phase |= dop.mat_size << kPhaseNormShift | (so.kind == SK_DIAG1 || so.kind == SK_DIAG2 ? kPhaseDiag : 0);
+                }
                 stage_ops.push_back(so);
             }
             sd.op_end = int(stage_ops.size()) - sop_begin;
