@@ -80,8 +80,8 @@ typedef struct mqb_gate_desc {
     int32_t pauli_ny;
     int32_t flags;                /* MQB_GATE_NONUNITARY: the constant matrix is not unitary (the
                                      superoperator of a noise channel on a vectorized density matrix):
-                                     it runs in a pass of its own, never inside a fused pass, and
-                                     gradients through it need checkpoint stride 1 */
+                                     it shares fused passes only with others like it, and gradients
+                                     through it need checkpoint stride 1 */
 } mqb_gate_desc;
 
 #define MQB_GATE_NONUNITARY 1

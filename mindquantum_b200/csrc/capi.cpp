@@ -222,7 +222,7 @@ struct mqb_program {
     int n_slots = 0;
     int32_t *d_csr_ptr = nullptr, *d_csr_slot = nullptr;
     double *d_csr_coeff = nullptr;
-    std::vector<char> no_fuse;   // per op: MQB_GATE_NONUNITARY
+    std::vector<char> apart;   // per op: MQB_GATE_NONUNITARY
     bool nonunitary = false;
     std::unique_ptr<SchedDev> apply_sched;
     std::map<int, std::unique_ptr<SchedDev>> grad_sched;   // by number of Hamiltonians
@@ -338,7 +338,7 @@ static std::unique_ptr<SchedDev> make_sched(const mqb_program &p, int K, bool fu
     // the register kernels need 2^5..2^8 threads of 2^reg_bits amplitudes: smaller registers use
     // the per-gate kernels
     if (K < reg_bits + 5) fuse = false;
-    sd->s = build_schedule(p.n, K, contiguity_bits(p.precision), p.ops, fuse, &p.no_fuse,
+    sd->s = build_schedule(p.n, K, contiguity_bits(p.precision), p.ops, fuse, &p.apart,
                            pass_limits(p, K, reg_bits, n_hams));
     build_stages(sd->s, p.ops, reg_bits, p.precision, false);
     build_stages(sd->s, p.ops, p.use_jit() ? jit_fwd_reg_bits(p.precision) : fwd_reg_bits(p.precision), p.precision, true);
@@ -484,10 +484,10 @@ static void apply_impl(mqb_program &p, void *states, int64_t batch, const double
     const size_t need = align_up(size_t(batch) * p.per_sample * sizeof(cplx<R>));
     if (p.per_sample && (ws == nullptr || ws_bytes < need)) fail(MQB_ERR_WORKSPACE, "workspace too small");
     cplx<R> *mats = static_cast<cplx<R> *>(ws);
-    run_matgen<R>(p, params, param_stride, custom, batch, mats, st);
     cplx<R> *s = static_cast<cplx<R> *>(states);
     SchedDev &sd = *p.apply_sched;
     if (runs_small(p, sd, batch)) {
+        run_matgen<R>(p, params, param_stride, custom, batch, mats, st);
         SmallArgs<R> a = small_args<R>(p, sd, mats, batch);
         a.src = s;
         a.src_stride = int64_t(1) << p.n;
@@ -497,6 +497,7 @@ static void apply_impl(mqb_program &p, void *states, int64_t batch, const double
         return;
     }
     const auto *jk = jit_forward(p, sd);
+    run_matgen<R>(p, params, param_stride, custom, batch, mats, st);
     for (size_t i = 0; i < sd.s.passes.size(); ++i)
         run_forward_pass<R>(p, sd, i, jk ? (*jk)[i] : nullptr, mats, s, int64_t(1) << p.n, s, batch, st);
 }
@@ -705,13 +706,13 @@ static void grad_impl(mqb_program &p, const mqb_hamiltonian *const *hams, int n_
         ++n_checked;
     };
     size_t next_fwd = 0, next_bwd = 0;
+    const auto *jf = jit_forward(p, sd);
+    const auto *jb = jit_backward(p, sd, n_hams);
     run_matgen<R>(p, params, param_stride, custom, batch, mats, st);
 
     // forward: psi_{q+1} = pass_q(psi_q), psi_0 = init (or |0...0>)
     const V *init_v = static_cast<const V *>(init);
     const int64_t init_stride = init_batched ? dim : 0;
-    const auto *jf = jit_forward(p, sd);
-    const auto *jb = jit_backward(p, sd, n_hams);
     for (int q = 0; q < P; ++q) {
         const V *src = (q == 0) ? init_v : loc(q);
         const int64_t sstr = (q == 0) ? init_stride : dim;
@@ -1018,11 +1019,11 @@ int mqb_program_create(int n_qubits, int precision, const mqb_gate_desc *gates, 
         p->tile_bits = options ? options->tile_bits : 0;
         p->jit = options ? options->jit : 0;
         p->descs.assign(gates, gates + n_gates);
-        p->no_fuse.assign(size_t(n_gates), 0);
+        p->apart.assign(size_t(n_gates), 0);
         for (int k = 0; k < n_gates; ++k)
             if (gates[k].flags & MQB_GATE_NONUNITARY) {
                 if (gates[k].gate_id != GID_MATRIX) fail(MQB_ERR_INVALID, "gate %d: only constant matrices can be non-unitary", k);
-                p->no_fuse[size_t(k)] = 1;
+                p->apart[size_t(k)] = 1;
                 p->nonunitary = true;
             }
         std::vector<std::complex<double>> pool;
@@ -1066,6 +1067,13 @@ int mqb_program_create(int n_qubits, int precision, const mqb_gate_desc *gates, 
                 slots += r;
             }
             p->ops.push_back(op);
+        }
+        uint64_t seen = 0;
+        for (DevOp &op : p->ops) {
+            uint64_t touch = op.ctrl | op.px | op.py | op.pz;
+            for (int i = 0; i < op.m; ++i) touch |= uint64_t(1) << op.tq[i];
+            if (op.unitary && !op.per_sample && !(seen & touch)) op.unitary = 2;
+            seen |= touch;
         }
         p->per_sample = cursor;
         p->n_slots = slots;

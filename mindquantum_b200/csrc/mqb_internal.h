@@ -43,7 +43,8 @@ struct DevOp {
     uint64_t px, py, pz;         // GID_RPS masks
     int32_t pny;
     int32_t sub;                 // dense single-qubit structure: SUB_GENERIC, SUB_REAL, SUB_PERM, SUB_SWAP, SUB_RXL
-    int32_t unitary;             // 1: unitary whatever its parameters (0: a custom gate or a matrix that is not)
+    int32_t unitary;             // 1: unitary whatever its parameters (0: a custom gate or a matrix that is not); 2: a
+                                 // unitary constant matrix, and the first gate on its qubits
     int32_t pad;
 };
 // Structure of a dense single-qubit matrix, used to pick a cheaper register kernel.
@@ -208,9 +209,9 @@ struct PassLimits {
 };
 
 // Builders (scheduler.cpp)
-// no_fuse (optional, one entry per op): ops that must run in a pass of their own.
+// apart (optional, one entry per op): non-unitary ops, which share passes only with one another.
 Schedule build_schedule(int n, int K, int c, const std::vector<DevOp> &ops, bool fuse,
-                        const std::vector<char> *no_fuse = nullptr, const PassLimits &limits = PassLimits());
+                        const std::vector<char> *apart = nullptr, const PassLimits &limits = PassLimits());
 // Split every fused pass of `s` into register stages with `reg_bits` register bits per thread:
 // the backward layout (Schedule::stages) or, with `forward`, the forward layout (f_stages).
 void build_stages(Schedule &s, const std::vector<DevOp> &ops, int reg_bits, int precision, bool forward = false);

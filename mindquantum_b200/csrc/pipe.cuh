@@ -136,7 +136,7 @@ __device__ __forceinline__ void pass_phase(V *ph, const V *mtab, const JitMtab *
         const int kind = e.phase & 3, norm = e.phase >> 8;
         double q = 1;   // mean square of what the gate multiplies amplitudes by
         auto sq = [&](int i) { return double(M[i].x) * double(M[i].x) + double(M[i].y) * double(M[i].y); };
-        if (kind == 1) p = reg::unit(reg::cmul(p, reg::wide(M[0])));
+        if (kind == 1) p = reg::cmul(p, reg::unit(reg::wide(M[0])));
         if (norm) {
             if (kind == 1) {            // (1, r)
                 q = 0.5 * (1.0 + sq(1));

@@ -87,27 +87,32 @@ struct ScanItem {
     uint64_t touch = 0, dense = 0;
     int slots = 0, entries = 0;
     bool fusable = true;
+    bool apart = false;              // runs only with others of its kind (a non-unitary operator)
 };
 
 struct ScanLimits {
     int K = 0;                       // qubits of the set
     int max_items = 1 << 30, max_slots = 1 << 30, max_entries = 1 << 30;
     uint64_t all = 0;
+    bool apart = false;              // the kind of items the set is for
 };
 
 // The items of `left` (indices, in program order) that can run together when the set is Q, which
 // grows up to K qubits as the items ask for them when `grow`.  An item that cannot join blocks the
-// qubits it touches for the rest of the scan.  Returns how many join; `members` may be null.
+// qubits it touches for the rest of the scan.  Returns how many join; `members` may be null; `wanted`
+// (optional) gets the qubits outside Q that kept an otherwise free item out.
 int scan_items(const std::vector<ScanItem> &items, const std::vector<int> &left, const ScanLimits &lim, uint64_t &Q,
-               bool grow, std::vector<int> *members) {
+               bool grow, std::vector<int> *members, uint64_t *wanted = nullptr) {
     uint64_t blocked = 0;
+    if (wanted) *wanted = 0;
     int n_items = 0, n_slots = 0, n_entries = 0;
     for (int i : left) {
         const ScanItem &it = items[i];
         if (n_items >= lim.max_items) break;
         const uint64_t need = it.dense & ~Q;
-        if ((it.touch & blocked) || !it.fusable || (need && (!grow || popc(Q | need) > lim.K)) ||
+        if ((it.touch & blocked) || !it.fusable || it.apart != lim.apart || (need && (!grow || popc(Q | need) > lim.K)) ||
             n_slots + it.slots > lim.max_slots || n_entries + it.entries > lim.max_entries) {
+            if (wanted && need && !(it.touch & blocked) && it.fusable && it.apart == lim.apart) *wanted |= need;
             blocked |= it.touch;
             if ((blocked & lim.all) == lim.all) break;
             continue;
@@ -147,22 +152,23 @@ uint64_t choose_set(const std::vector<ScanItem> &items, const std::vector<int> &
             if (popc(Q) == lim.K) offer(Q, scan_items(items, left, lim, Q, false, nullptr));
         }
     }
-    uint64_t Q = Q0;
-    int got = scan_items(items, left, lim, Q, false, nullptr);
-    while (popc(Q) < lim.K) {
+    uint64_t Q = Q0, wanted = 0;
+    int got = scan_items(items, left, lim, Q, false, nullptr, &wanted);
+    while (popc(Q) < lim.K && wanted) {   // only a wanted qubit lets more items join
         int step_got = -1;
-        uint64_t step_q = Q;
-        for (int q = 0; q < n; ++q) {
-            if (Q >> q & 1) continue;
-            uint64_t t = Q | uint64_t(1) << q;
-            const int g = scan_items(items, left, lim, t, false, nullptr);
+        uint64_t step_q = Q, step_wanted = 0;
+        for (uint64_t rest = wanted; rest; rest &= rest - 1) {
+            uint64_t t = Q | (rest & ~(rest - 1)), w = 0;
+            const int g = scan_items(items, left, lim, t, false, nullptr, &w);
             if (g > step_got) {
                 step_got = g;
                 step_q = t;
+                step_wanted = w;
             }
         }
         Q = step_q;
         got = step_got;
+        wanted = step_wanted;
     }
     offer(Q, got);
     return best_q;
@@ -176,7 +182,7 @@ struct Cut {
 };
 
 // Cut the items into groups, each group's set taken in program order or, with `search`, by choose_set.
-std::vector<Cut> cut_items(const std::vector<ScanItem> &items, const ScanLimits &lim, uint64_t Q0, int n, bool windows,
+std::vector<Cut> cut_items(const std::vector<ScanItem> &items, ScanLimits lim, uint64_t Q0, int n, bool windows,
                            bool search) {
     std::vector<int> left(items.size()), rest;
     for (size_t i = 0; i < items.size(); ++i) left[i] = int(i);
@@ -185,6 +191,7 @@ std::vector<Cut> cut_items(const std::vector<ScanItem> &items, const ScanLimits 
         Cut c;
         if (items[size_t(left.front())].fusable) {
             c.set = Q0;
+            lim.apart = items[size_t(left.front())].apart;
             if (search) c.set = choose_set(items, left, lim, Q0, n, windows);
             scan_items(items, left, lim, c.set, !search, &c.members);
         }
@@ -211,9 +218,8 @@ std::vector<Cut> best_cut(const std::vector<ScanItem> &items, const ScanLimits &
 
 }  // namespace
 
-Schedule build_schedule(int n, int K, int c, const std::vector<DevOp> &ops, bool fuse, const std::vector<char> *no_fuse,
+Schedule build_schedule(int n, int K, int c, const std::vector<DevOp> &ops, bool fuse, const std::vector<char> *apart,
                         const PassLimits &limits) {
-    auto fusable_at = [&](int i) { return fusable(ops[i]) && !(no_fuse && (*no_fuse)[i]); };
     Schedule s;
     if (K > n) K = n;
     // leave room for the widest fused gate next to the contiguity bits; keep at least one
@@ -231,7 +237,8 @@ Schedule build_schedule(int n, int K, int c, const std::vector<DevOp> &ops, bool
         it.dense = dense_targets(ops[i]);
         it.slots = popc(uint64_t(ops[i].grad_mask));
         it.entries = ops[i].mat_size * (1 + (limits.derivatives && ops[i].grad_mask ? ops[i].n_angles : 0));
-        it.fusable = fuse && fusable_at(i);
+        it.fusable = fuse && fusable(ops[i]);
+        it.apart = apart && (*apart)[i];
     }
     ScanLimits lim;
     lim.K = K;
@@ -538,7 +545,9 @@ void build_stages(Schedule &s, const std::vector<DevOp> &ops, int reg_bits, int 
                     else if (zz && (reg0 || reg1) && !so.rctrl)
                         so.phase |= kPhasePair;
                     if (zz && reg0 && reg1 && dop.ctrl && !so.rctrl) so.phase |= kPhasePair;
-                    if (precision == MQB_PREC_C64 && !dop.ctrl && so.kind != SK_SWAP1) so.phase |= dop.mat_size << kPhaseNormShift | (so.kind == SK_DIAG1 || so.kind == SK_DIAG2 ? kPhaseDiag : 0);
+                    // (of the constant matrices only the first gate on a qubit counts: on the structured states of
+                    // Clifford circuits the roundings of later ones cancel)
+                    if (precision == MQB_PREC_C64 && !dop.ctrl && so.kind != SK_SWAP1 && (dop.per_sample || dop.unitary == 2)) so.phase |= dop.mat_size << kPhaseNormShift | (so.kind == SK_DIAG1 || so.kind == SK_DIAG2 ? kPhaseDiag : 0);
                 }
                 stage_ops.push_back(so);
             }
