@@ -10,7 +10,7 @@ engine: column index j on qubits 0..n-1, row index i on qubits n..2n-1.  Then
   the fused pass kernels unchanged;
 * a channel becomes its superoperator, sum_k K_k (x) conj(K_k) on (q + n, q), or the reference's
   direct map for depolarizing and thermal relaxation (cpu_densitymatrix_core_channel.cpp); these
-  are non-unitary constant matrices that run in passes of their own;
+  are non-unitary constant matrices that share passes only with one another;
 * Tr(H rho) = <vec(H)|vec(rho)>, with vec(H) = (H (x) I) vec(I) made by the Hamiltonian kernels;
 * the gradient of Tr(H E(rho_0)) is linear in vec(rho): it is the adjoint sweep with the given
   lambda = vec(H) (mqb_adjoint_with_lambda, Re sum <lambda|dS|rho>), where the row and column
@@ -37,7 +37,7 @@ from .lowering import lowered, native_ham
 from .measure_result import MeasureResult
 from .mqvector_b200 import MQVectorB200, _ptr, _split_inputs, _stream
 from .rng import Mt19937Uniform
-from .utils import GradOpsWrapper, check_kept_qubits, qs_of_qubits
+from .utils import GradOpsWrapper, KeptCircuits, check_kept_qubits, qs_of_qubits
 
 _CHANNEL_NAMES = ('PC', 'BFC', 'PFC', 'BPFC', 'GPC', 'DC', 'ADC', 'PDC', 'TRC')
 # conj(exp(-i t/2 G)) = exp(-i (-t)/2 G) when the generator G is real, itself when G is imaginary
@@ -202,6 +202,7 @@ class MQMatrixB200(BackendBase):
         self.seed = seed
         self.engine = MQVectorB200(name, 2 * n_qubits, seed, self.arithmetic_type, fuse, device, jit)
         self._ham_vec = {}
+        self._doubled_kept = KeptCircuits()
         self._rng = Mt19937Uniform(seed)   # the measurement stream of apply_circuit
 
     # ------------------------------------------------------------------ state
@@ -336,6 +337,11 @@ class MQMatrixB200(BackendBase):
             N.call('mqb_apply_hamiltonian', h.handle, _ptr(self.engine.state), _ptr(out), 1, _stream())
             self.engine.set_state_tensor(out)
 
+    def _doubled(self, circ):
+        """``doubled_circuit`` of a circuit, the last few kept with their lowered programs (doubling and
+        lowering 56 gates anew takes 4 ms)."""
+        return self._doubled_kept.get(circ, lambda c: doubled_circuit(c, self.n_qubits))
+
     # ------------------------------------------------------------------ expectations
     def _vec_h(self, ham):
         """vec(H) = (H (x) I) vec(I) on the doubled register (cached per Hamiltonian object)."""
@@ -372,7 +378,7 @@ class MQMatrixB200(BackendBase):
         st = self.engine.state.clone()
         if circ_right is not None and len(circ_right):
             pr = self.engine._check_pr(circ_right, pr)   # pylint: disable=protected-access
-            dc = doubled_circuit(circ_right, self.n_qubits)
+            dc = self._doubled(circ_right)
             if len(dc):
                 self.engine._apply_segment(st, dc, pr)   # pylint: disable=protected-access
         o = self._expect(hamiltonian, st.reshape(1, -1)).cpu().numpy()
@@ -382,7 +388,7 @@ class MQMatrixB200(BackendBase):
         """f [batch][n_hams] and grad [batch][n_hams][n_params] (float64 device tensors) of Tr(H E(rho))."""
         params = params.to(device=self.device, dtype=torch.float64).contiguous()
         B = params.shape[0]
-        dc = doubled_circuit(circuit, self.n_qubits)
+        dc = self._doubled(circuit)
         names = list(param_names)
         prog = lowered(dc, 2 * self.n_qubits, self.precision, names, None, self.engine.fuse, jit=self.engine.jit)
         init = self.engine.state
@@ -391,16 +397,13 @@ class MQMatrixB200(BackendBase):
         states = self.engine._batched_states(dc, names, init, params)   # pylint: disable=protected-access
         custom = self.engine._custom_tensor(prog, params.cpu().numpy()) if prog.customs else None  # pylint: disable=protected-access
         has_channel = any(getattr(x, 'nonunitary', False) for x in dc)
-        stride = 1 if has_channel else self.engine._choose_stride(prog, B, 1)   # pylint: disable=protected-access
-        ws_bytes = ctypes.c_size_t()
-        N.call('mqb_grad_workspace_size', prog.handle, B, 1, stride, ctypes.byref(ws_bytes))
-        ws = torch.empty(max(256, ws_bytes.value), dtype=torch.uint8, device=self.device)
+        stride, ws = self.engine._grad_workspace(prog, B, 1, 1 if has_channel else None, 256)   # pylint: disable=protected-access
         for h, ham in enumerate(hams):
             f[:, h] = self._expect(ham, states)[:, 0]
             lam = self._vec_h(ham)
             gh = torch.zeros((B, max(1, len(names))), dtype=torch.float64, device=self.device)
             N.call('mqb_adjoint_with_lambda', prog.handle, _ptr(lam), 0, _ptr(init), 0, B, _ptr(params),
-                   params.shape[1], _ptr(custom), _ptr(gh), stride, _ptr(ws), ws_bytes.value, _stream())
+                   params.shape[1], _ptr(custom), _ptr(gh), stride, _ptr(ws), ws.numel(), _stream())
             g[:, h] = gh
         return f, g[:, :, :len(names)]
 
