@@ -216,6 +216,7 @@ struct mqb_program {
     mqb_gate_desc *d_descs = nullptr;
     mqb_param_term *d_terms = nullptr;
     void *d_cpool = nullptr;
+    void *d_cpool64 = nullptr;   // the pool in FP64 (d_cpool itself in complex128)
     int64_t n_pool = 0;        // complex entries of the constant pool
     int64_t per_sample = 0;    // complex entries per sample
     int64_t custom_entries = 0;
@@ -231,6 +232,7 @@ struct mqb_program {
         cudaFree(d_descs);
         cudaFree(d_terms);
         cudaFree(d_cpool);
+        if (d_cpool64 != d_cpool) cudaFree(d_cpool64);
         cudaFree(d_csr_ptr);
         cudaFree(d_csr_slot);
         cudaFree(d_csr_coeff);
@@ -280,6 +282,10 @@ static PassLimits pass_limits(const mqb_program &p, int K, int reg_bits, int n_h
     PassLimits lim;
     lim.max_entries = int(std::max<int64_t>(bytes, 4096) / int64_t(p.elem()));
     lim.derivatives = n_hams > 0;
+    // Searched sets reorder gates, which in complex64 moves an expectation of 1e-2 by 1e-5 of itself; it pays
+    // where passes cost (generated kernels) and is free of that in complex128 (16 qubits x 8 layers: 7 -> 4
+    // passes, 0.67 -> 0.60 ms), but the precompiled complex64 kernels of smaller registers gain little.
+    lim.search = p.use_jit() || p.precision == MQB_PREC_C128;
     return lim;
 }
 
@@ -302,7 +308,7 @@ static void plan_small(const mqb_program &p, SchedDev &sd, int n_hams) {
     if (n_hams > 0 && p.nonunitary) return;
     for (const DevOp &op : p.ops)
         if (op.kind == KIND_RPS || op.m > kMaxFusedM) return;
-    const size_t smem = small_smem(p.n, int(p.elem()), n_hams, int(p.ops.size()), p.per_sample + p.n_pool, n_hams ? p.n_slots : 0);
+    const size_t smem = small_smem(p.n, n_hams ? int(sizeof(double2)) : int(p.elem()), n_hams, int(p.ops.size()), p.per_sample + p.n_pool, n_hams ? p.n_slots : 0);
     if (!smem) return;
     std::vector<SmallOp> v;
     const int P = int(sd.s.passes.size()), sn = norm_stride(P);
@@ -452,6 +458,7 @@ static void run_matgen(const mqb_program &p, const double *params, int64_t param
     m.batch = batch;
     m.mats = mats;
     m.mats_stride = p.per_sample;
+    m.ratios = p.use_jit();
     TimeScope ts(TK_MATGEN, st);
     ck(launch_matgen<R>(m, st), "matgen");
 }
@@ -464,15 +471,16 @@ static bool runs_small(const mqb_program &p, const SchedDev &sd, int64_t batch) 
     return !tiles || p.n <= kSmallAnyBatchQubits || batch <= 2 * int64_t(sm_count_cached());
 }
 
-template <typename R>
-static SmallArgs<R> small_args(const mqb_program &p, const SchedDev &sd, const cplx<R> *mats, int64_t batch) {
-    SmallArgs<R> a{};
+template <typename R, typename S>
+static SmallArgs<R, S> small_args(const mqb_program &p, const SchedDev &sd, const cplx<R> *mats, const void *cpool,
+                                  int64_t batch) {
+    SmallArgs<R, S> a{};
     a.n = p.n;
     a.n_ops = int(p.ops.size());
     a.ops = sd.d_small;
     a.mats = mats;
     a.mats_stride = p.per_sample;
-    a.cpool = static_cast<const cplx<R> *>(p.d_cpool);
+    a.cpool = static_cast<const cplx<R> *>(cpool);
     a.n_pool = int(p.n_pool);
     a.batch = batch;
     return a;
@@ -488,12 +496,12 @@ static void apply_impl(mqb_program &p, void *states, int64_t batch, const double
     SchedDev &sd = *p.apply_sched;
     if (runs_small(p, sd, batch)) {
         run_matgen<R>(p, params, param_stride, custom, batch, mats, st);
-        SmallArgs<R> a = small_args<R>(p, sd, mats, batch);
+        SmallArgs<R, R> a = small_args<R, R>(p, sd, mats, p.d_cpool, batch);
         a.src = s;
         a.src_stride = int64_t(1) << p.n;
         a.dst = s;
         TimeScope ts(TK_FWD, st);
-        ck(launch_small<R>(a, sd.small_smem, st), "small register");
+        ck((launch_small<R, R>(a, sd.small_smem, st)), "small register");
         return;
     }
     const auto *jk = jit_forward(p, sd);
@@ -608,7 +616,7 @@ struct GradLayout {
     std::vector<int> norm_fwd, norm_bwd;
 };
 
-static GradLayout grad_layout(const mqb_program &p, const Schedule &s, int64_t batch, int n_hams, int stride) {
+static GradLayout grad_layout(const mqb_program &p, const Schedule &s, int64_t batch, int n_hams, int stride, bool small) {
     GradLayout L;
     const int P = int(s.passes.size());
     const size_t state = (size_t(1) << p.n) * p.elem() * batch;
@@ -629,7 +637,7 @@ static GradLayout grad_layout(const mqb_program &p, const Schedule &s, int64_t b
         for (int q = P - 1; q >= 1; --q)
             if (L.ckpt_index[q] < 0 && q % sn == 0) L.norm_bwd.push_back(q);
     }
-    L.mats = align_up(size_t(batch) * p.per_sample * p.elem());
+    L.mats = align_up(size_t(batch) * p.per_sample * (small ? sizeof(double2) : p.elem()));
     L.gslots = align_up(size_t(batch) * std::max(1, p.n_slots) * n_hams * sizeof(double));
     L.lam = align_up(state * n_hams);
     L.w = L.need_w ? align_up(state) : 0;
@@ -653,7 +661,7 @@ static void grad_impl(mqb_program &p, const mqb_hamiltonian *const *hams, int n_
              stride);
     SchedDev &sd = grad_schedule(p, n_hams);
     const Schedule &s = sd.s;
-    const GradLayout L = grad_layout(p, s, batch, n_hams, stride);
+    const GradLayout L = grad_layout(p, s, batch, n_hams, stride, sd.small_smem != 0);
     if (ws == nullptr || ws_bytes < L.total) fail(MQB_ERR_WORKSPACE, "workspace too small (%zu < %zu)", ws_bytes, L.total);
     unsigned char *base = static_cast<unsigned char *>(ws);
     V *mats = reinterpret_cast<V *>(base);
@@ -670,8 +678,9 @@ static void grad_impl(mqb_program &p, const mqb_hamiltonian *const *hams, int n_
     const V *cpool = static_cast<const V *>(p.d_cpool);
 
     if (runs_small(p, sd, batch) && std::none_of(hams, hams + (lam_in ? 0 : n_hams), [](const mqb_hamiltonian *h) { return h->csr; })) {
-        run_matgen<R>(p, params, param_stride, custom, batch, mats, st);
-        SmallArgs<R> a = small_args<R>(p, sd, mats, batch);
+        cplx<double> *wide = reinterpret_cast<cplx<double> *>(base);   // FP64 whatever the caller's precision
+        run_matgen<double>(p, params, param_stride, custom, batch, wide, st);
+        SmallArgs<double, R> a = small_args<double, R>(p, sd, wide, p.d_cpool64, batch);
         a.src = static_cast<const V *>(init);
         a.src_stride = init_batched ? dim : 0;
         a.n_hams = n_hams;
@@ -691,7 +700,7 @@ static void grad_impl(mqb_program &p, const mqb_hamiltonian *const *hams, int n_
         a.norms = L.norms ? reinterpret_cast<double *>(ck0 + L.ckpt) : nullptr;
         a.ckpt_stride = stride;
         TimeScope ts(TK_BWD, st);
-        ck(launch_small<R>(a, sd.small_smem, st), "small register gradient");
+        ck((launch_small<double, R>(a, sd.small_smem, st)), "small register gradient");
         return;
     }
     ck(cudaMemsetAsync(gslots, 0, L.gslots, st), "memset");
@@ -1082,14 +1091,15 @@ int mqb_program_create(int n_qubits, int precision, const mqb_gate_desc *gates, 
         p->d_terms = upload(std::vector<mqb_param_term>(terms, terms + n_terms));
         p->n_pool = int64_t(pool.size());
         if (!pool.empty()) {
+            std::vector<double2> wide;
+            for (auto &c : pool) wide.push_back(make_double2(c.real(), c.imag()));
             if (precision == MQB_PREC_C64) {
                 std::vector<float2> v;
                 for (auto &c : pool) v.push_back(make_float2(float(c.real()), float(c.imag())));
                 p->d_cpool = upload(v);
+                if (n_qubits <= kSmallMaxQubits) p->d_cpool64 = upload(wide);
             } else {
-                std::vector<double2> v;
-                for (auto &c : pool) v.push_back(make_double2(c.real(), c.imag()));
-                p->d_cpool = upload(v);
+                p->d_cpool64 = p->d_cpool = upload(wide);
             }
         }
         std::vector<int32_t> ptr(std::max(0, n_params) + 1, 0), slot;
@@ -1487,7 +1497,7 @@ int mqb_grad_workspace_size(const mqb_program *p, int64_t batch, int n_hams, int
         if (n_hams < 1) fail(MQB_ERR_INVALID, "need at least one Hamiltonian");
         if (batch < 1) fail(MQB_ERR_INVALID, "batch must be >= 1");
         SchedDev &sd = grad_schedule(const_cast<mqb_program &>(*p), n_hams);
-        *bytes = grad_layout(*p, sd.s, batch, n_hams, stride).total;
+        *bytes = grad_layout(*p, sd.s, batch, n_hams, stride, sd.small_smem != 0).total;
     });
 }
 
@@ -1498,7 +1508,7 @@ int mqb_grad_norm_checks(mqb_program *p, const void *ws, size_t ws_bytes, int64_
         if (!p || !n_checks) fail(MQB_ERR_INVALID, "null argument");
         if (n_hams < 1 || batch < 1) fail(MQB_ERR_INVALID, "invalid batch or number of Hamiltonians");
         SchedDev &sd = grad_schedule(*p, n_hams);
-        const GradLayout L = grad_layout(*p, sd.s, batch, n_hams, stride);
+        const GradLayout L = grad_layout(*p, sd.s, batch, n_hams, stride, sd.small_smem != 0);
         const int n = int(L.norm_fwd.size() + L.norm_bwd.size());
         *n_checks = n;
         if (n == 0 || !out) return;

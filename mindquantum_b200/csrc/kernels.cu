@@ -320,7 +320,7 @@ __global__ void matgen_kernel(MatgenArgs a) {
         }
         GateMats gm;
         gate_mats(op.gate_id, t, gm);
-        if (sizeof(R) == 4 && (op.gate_id == GID_RZ || op.gate_id == GID_RZZ)) {
+        if (sizeof(R) == 4 && a.ratios && (op.gate_id == GID_RZ || op.gate_id == GID_RZZ)) {
             // what the state sees is the ratio of the two phases, e^{i t}: take the second from the rounded first, so
             // that complex64 rounds the ratio once instead of twice the half angle
             const double ar = double(float(gm.M[0].x)), ai = double(float(gm.M[0].y));

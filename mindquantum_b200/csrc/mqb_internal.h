@@ -151,6 +151,7 @@ struct Pass {
 
 struct Schedule {
     int K = 0;
+    bool search = true;             // PassLimits::search, for the stages too
     std::vector<Pass> passes;
     std::vector<PassOp> pass_ops;
     std::vector<int32_t> slot_map;  // pass-local slot -> global gradient slot
@@ -206,6 +207,7 @@ class JitBlock {
 struct PassLimits {
     int max_entries = 1 << 30;   // complex entries of the pass's shared-memory matrix table
     bool derivatives = true;     // whether the table holds the gates' derivative matrices too
+    bool search = true;          // search the sets (else program order)
 };
 
 // Builders (scheduler.cpp)

@@ -209,9 +209,10 @@ std::vector<Cut> cut_items(const std::vector<ScanItem> &items, ScanLimits lim, u
 }
 
 // The cut with fewer groups; program order where the search saves none (its groups are more even).
-std::vector<Cut> best_cut(const std::vector<ScanItem> &items, const ScanLimits &lim, uint64_t Q0, int n, bool windows) {
+std::vector<Cut> best_cut(const std::vector<ScanItem> &items, const ScanLimits &lim, uint64_t Q0, int n, bool windows,
+                          bool search) {
     std::vector<Cut> plain = cut_items(items, lim, Q0, n, windows, false);
-    if (n <= lim.K || plain.size() < 3) return plain;
+    if (!search || n <= lim.K || plain.size() < 3) return plain;
     std::vector<Cut> found = cut_items(items, lim, Q0, n, windows, true);
     return found.size() < plain.size() ? found : plain;
 }
@@ -228,6 +229,7 @@ Schedule build_schedule(int n, int K, int c, const std::vector<DevOp> &ops, bool
     if (n > K && K < kMaxFusedM + 1) fuse = false;
     if (K < 6) fuse = false;
     s.K = K;
+    s.search = limits.search;
     const int L = int(ops.size());
     const uint64_t all = n >= 64 ? ~uint64_t(0) : ((uint64_t(1) << n) - 1);
     std::vector<ScanItem> items(static_cast<size_t>(L));
@@ -246,7 +248,7 @@ Schedule build_schedule(int n, int K, int c, const std::vector<DevOp> &ops, bool
     lim.max_slots = kMaxPassSlots;
     lim.max_entries = limits.max_entries;
     lim.all = all;
-    for (const Cut &cut : best_cut(items, lim, (n <= K) ? all : ((uint64_t(1) << c) - 1), n, true)) {
+    for (const Cut &cut : best_cut(items, lim, (n <= K) ? all : ((uint64_t(1) << c) - 1), n, true, limits.search)) {
         const std::vector<int> &members = cut.members;
         if (cut.single) {
             const int first = members.front();
@@ -434,7 +436,7 @@ void build_stages(Schedule &s, const std::vector<DevOp> &ops, int reg_bits, int 
         ScanLimits lim;
         lim.K = RB;
         lim.all = (uint64_t(1) << K) - 1;
-        for (const Cut &cut : best_cut(items, lim, 0, K, false)) {
+        for (const Cut &cut : best_cut(items, lim, 0, K, false, s.search)) {
             const std::vector<int> &members = cut.members;
             // keep only the bits that a member needs: the rest is padded below
             uint32_t R = 0;

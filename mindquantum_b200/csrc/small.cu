@@ -9,7 +9,8 @@
 // the smallest registers ran one kernel per gate (a 6-qubit classifier's training step on 32 samples: 310
 // launches), and those of a single tile ran one block's serial chain of 16 to 32 amplitudes
 // per thread in several launches.  Here a gate costs a shared-memory round trip of one pair per thread
-// and a barrier, which is what bounds it: latency, not throughput.
+// and a barrier, which is what bounds it: latency, not throughput.  So a complex64 gradient runs in FP64 here
+// (10 qubits, 4 Hamiltonians, one sample: 298 us against 277), its caller's states converted on the way in.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -82,8 +83,16 @@ __device__ __forceinline__ void gate2(const SmallOp &op, const V *M, V (&x)[4]) 
     for (int r = 0; r < 4; ++r) x[r] = y[r];
 }
 
-template <typename R>
-__global__ void __launch_bounds__(kSmallThreads) small_kernel(const SmallArgs<R> a) {
+template <typename V, typename W>
+__device__ __forceinline__ V as(W a) {
+    V r;
+    r.x = a.x;
+    r.y = a.y;
+    return r;
+}
+
+template <typename R, typename S>
+__global__ void __launch_bounds__(kSmallThreads) small_kernel(const SmallArgs<R, S> a) {
     using V = cplx<R>;
     extern __shared__ __align__(16) unsigned char smem[];
     const int n = a.n, T = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = T >> 5;
@@ -111,7 +120,7 @@ __global__ void __launch_bounds__(kSmallThreads) small_kernel(const SmallArgs<R>
             V v;
             v.x = i == 0;
             v.y = 0;
-            psi[i] = a.src ? a.src[b * a.src_stride + i] : v;
+            psi[i] = a.src ? as<V>(a.src[b * a.src_stride + i]) : v;
         }
     }
     __syncthreads();
@@ -163,13 +172,13 @@ __global__ void __launch_bounds__(kSmallThreads) small_kernel(const SmallArgs<R>
         if (a.norms && (op.check & 1)) norm_check();
     }
     if (a.dst)
-        for (unsigned i = tid; i < dim; i += T) a.dst[b * dim + i] = psi[i];
+        for (unsigned i = tid; i < dim; i += T) a.dst[b * dim + i] = as<cplx<S>>(psi[i]);
     if (NH == 0) return;
     // lambda_h = H_h psi and f_h = <psi|lambda_h>, sums in FP64
     for (int h = 0; h < NH; ++h) {
         V *lh = lam + size_t(h) * dim;
         if (a.lam_in) {
-            for (unsigned i = tid; i < dim; i += T) lh[i] = a.lam_in[b * a.lam_stride + i];
+            for (unsigned i = tid; i < dim; i += T) lh[i] = as<V>(a.lam_in[b * a.lam_stride + i]);
             continue;
         }
         const SmallHam &H = a.ham[h];
@@ -339,15 +348,16 @@ size_t small_smem(int n, int elem_bytes, int n_hams, int n_ops, int64_t table_en
     return s <= (size_t(200) << 10) ? s : 0;
 }
 
-template <typename R>
-cudaError_t launch_small(const SmallArgs<R> &a, size_t smem, cudaStream_t s) {
-    cudaError_t e = cudaFuncSetAttribute(small_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+template <typename R, typename S>
+cudaError_t launch_small(const SmallArgs<R, S> &a, size_t smem, cudaStream_t s) {
+    cudaError_t e = cudaFuncSetAttribute(small_kernel<R, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
-    small_kernel<R><<<unsigned(a.batch), small_threads(a.n), smem, s>>>(a);
+    small_kernel<R, S><<<unsigned(a.batch), small_threads(a.n), smem, s>>>(a);
     return cudaGetLastError();
 }
 
-template cudaError_t launch_small<float>(const SmallArgs<float> &, size_t, cudaStream_t);
-template cudaError_t launch_small<double>(const SmallArgs<double> &, size_t, cudaStream_t);
+template cudaError_t launch_small<float, float>(const SmallArgs<float, float> &, size_t, cudaStream_t);
+template cudaError_t launch_small<double, float>(const SmallArgs<double, float> &, size_t, cudaStream_t);
+template cudaError_t launch_small<double, double>(const SmallArgs<double, double> &, size_t, cudaStream_t);
 
 }  // namespace mqb

@@ -27,7 +27,8 @@ struct SmallHam {
     int n_classes;
 };
 
-template <typename R>
+// R: the arithmetic; S: the caller's states.
+template <typename R, typename S = R>
 struct SmallArgs {
     int n, n_ops;
     const SmallOp *ops;
@@ -35,14 +36,14 @@ struct SmallArgs {
     int64_t mats_stride;
     const cplx<R> *cpool;
     int n_pool;
-    const cplx<R> *src;          // nullptr: |0...0>
+    const cplx<S> *src;          // nullptr: |0...0>
     int64_t src_stride;
-    cplx<R> *dst;                // apply: the final state; gradient: nullptr
+    cplx<S> *dst;                // apply: the final state; gradient: nullptr
     int64_t batch;
     // gradient
     int n_hams;
     SmallHam ham[kSmallMaxHams];
-    const cplx<R> *lam_in;       // lambda from the caller instead of the Hamiltonians (n_hams = 1)
+    const cplx<S> *lam_in;       // lambda from the caller instead of the Hamiltonians (n_hams = 1)
     int64_t lam_stride;
     double *f;                   // [batch][n_hams][2]
     double *grad;                // [batch][n_hams][n_params]
@@ -56,8 +57,8 @@ struct SmallArgs {
 
 // Shared memory of a block; 0 when the evaluation does not fit the kernel.
 size_t small_smem(int n, int elem_bytes, int n_hams, int n_ops, int64_t table_entries, int n_slots);
-template <typename R>
-cudaError_t launch_small(const SmallArgs<R> &a, size_t smem, cudaStream_t s);
+template <typename R, typename S>
+cudaError_t launch_small(const SmallArgs<R, S> &a, size_t smem, cudaStream_t s);
 
 }  // namespace mqb
 
