@@ -182,19 +182,20 @@ std::string lit(double x) {
 }
 
 // Gradient partials of an adjoint kernel.  A thread's partial of one (angle, Hamiltonian) is a row of its
-// warp's shared scratch; every kRowBatch rows the warp adds them up together (pipe::rows_flush_as): 5
-// instructions per row instead of 16 for a shuffle tree per partial, which was 30 to 40 % of the adjoint passes
-// (26-qubit ansatz, batch 2: 36.6 ms with the trees, 25.9 with no reduction at all).
+// warp's shared scratch; every `batch` rows the warp adds them up together (pipe::rows_flush_as): 5
+// instructions per row with four rows, 3.5 with eight, instead of 16 for a shuffle tree per partial, which was
+// 30 to 40 % of the adjoint passes (26-qubit ansatz, batch 2: 36.6 ms with the trees, 25.9 with no reduction
+// at all).  Eight rows against four: 31.6 to 30.7 ms on that ansatz, 30.1 to 28.4 on a 20-qubit network of
+// 512 samples.
 // Rows come in the order the kernel makes them; `order` maps them to pass-local slots.
-int row_batch(int precision) { return precision == MQB_PREC_C64 ? 4 : 2; }
-
 struct Rows {
     int batch = 4, NH = 1;
     std::vector<int> order;   // row -> lslot * NH + h
 
     void flush(std::ostringstream &o) const {
         const int n = int(order.size()) % batch == 0 ? batch : int(order.size()) % batch;
-        o << "    pipe::rows_flush_as<R>(scr, wrow + " << int(order.size()) - n << ", " << n << ", lane);\n";
+        o << "    pipe::rows_flush_as<R, " << batch << ">(scr, wrow + " << int(order.size()) - n << ", " << n
+          << ", lane);\n";
     }
     // the partial `expr` of slot lslot and Hamiltonian h
     void put(std::ostringstream &o, const std::string &expr, int lslot, int h) {
@@ -835,25 +836,32 @@ int bwd_groups(const Pass &p) {
     return std::min(max_groups(nt), env_int("MQB_PIPE_BWD_GROUPS", 2, 1, 15));
 }
 
-size_t bwd_fixed_smem(const Pass &p, int precision, int n_hams) {
+size_t bwd_fixed_smem(const Pass &p, int precision, int n_hams, int scratch) {
     const size_t eb = elem_bytes(precision);
     const int nw = (1 << (p.K - p.reg_bits)) / 32;
     return size_t(bwd_groups(p)) *
                (a16(size_t(p.mtab_entries) * eb) + a16(size_t(nw) * std::max(1, p.n_slots) * n_hams * sizeof(double)) +
-                size_t(nw) * 512) +
+                size_t(nw) * size_t(scratch)) +
            8 * 16 + 16 * size_t(eb);
 }
 
-// Buffers of the adjoint ring: G + 1 where they fit in 227 KB, else as many as fit (at least G).
-int bwd_buffers(const Pass &p, int precision, int n_hams) {
+// Buffers of the adjoint ring: G + 1 where they fit in 227 KB, else as many as fit (at least G); 0: fewer than
+// G fit.
+int bwd_buffers(const Pass &p, int precision, int n_hams, int scratch) {
     const size_t buf = (size_t(1) << p.K) * elem_bytes(precision) * (1 + n_hams);
-    const size_t fixed = bwd_fixed_smem(p, precision, n_hams);
+    const size_t fixed = bwd_fixed_smem(p, precision, n_hams, scratch);
     const int G = bwd_groups(p);
     int nb = env_int("MQB_PIPE_BWD_BUFFERS", G + 1, 1, 8);
     while (nb > G && nb * buf + fixed > size_t(227) << 10) --nb;
-    if (nb * buf + fixed > size_t(227) << 10)
-        throw std::runtime_error("generated adjoint pass: the tile ring does not fit in shared memory");
-    return nb;
+    return nb * buf + fixed > size_t(227) << 10 ? 0 : nb;
+}
+
+// Bytes of gradient-row scratch per warp: four rows (two in complex128), or eight complex64 rows where they
+// cost the ring no buffer.
+int bwd_scratch(const Pass &p, int precision, int n_hams) {
+    const int nb = bwd_buffers(p, precision, n_hams, 512);
+    if (nb == 0) throw std::runtime_error("generated adjoint pass: the tile ring does not fit in shared memory");
+    return precision == MQB_PREC_C64 && bwd_buffers(p, precision, n_hams, 1024) == nb ? 1024 : 512;
 }
 
 void emit_header(std::ostringstream &o, int precision) {
@@ -1069,14 +1077,15 @@ std::string backward_source(const Schedule &s, const Pass &p, int precision, int
     const int RB = p.reg_bits, K = p.K, TB = K - RB;
     const int NLS = std::max(1, p.n_slots);
     const PassPlan pl = pass_plan(p.qbits, precision);
-    const int NB = bwd_buffers(p, precision, NH), G = bwd_groups(p);
+    const int scratch = bwd_scratch(p, precision, NH), NB = bwd_buffers(p, precision, NH, scratch);
+    const int G = bwd_groups(p);
     std::vector<const StageDesc *> ex;
     for (int si = p.n_stages - 1; si >= 0; --si) ex.push_back(&s.stages[p.stage_begin + si]);
     const LayPlan lp = plan_layouts(pl, ex, TB);
     bool pass_phase = false;
     for (int k = 0; k < p.n_sops; ++k) pass_phase = pass_phase || leaves_factor(s.stage_ops[p.sop_begin + k]);
     Rows rows;
-    rows.batch = row_batch(precision);
+    rows.batch = scratch / (32 * elem_bytes(precision) / 2);
     rows.NH = NH;
     std::ostringstream o;
     o << "extern \"C\" __global__ void __launch_bounds__(" << G * (1 << TB) << ", 1) mqb_adj_pass(const JitBwdArgs<V> a, "
@@ -1105,7 +1114,8 @@ std::string backward_source(const Schedule &s, const Pass &p, int precision, int
     o << "  const int warp = int(tid) / 32, lane = int(tid) % 32;\n"
       << "  V *mt = reinterpret_cast<V *>(smem + NB * BUFB + grp * mtb);\n"
       << "  double *wacc = wacc0 + grp * WS, *wrow = wacc + warp * NLS * NH;\n"
-      << "  const unsigned scr = pipe::saddr(reinterpret_cast<V *>(full + 16) + 16) + unsigned(grp * nw + warp) * 512u;\n"
+      << "  const unsigned scr = pipe::saddr(reinterpret_cast<V *>(full + 16) + 16) + unsigned(grp * nw + warp) * "
+      << scratch << "u;\n"
       << "  long long cached_b = -1;\n"
       << "  for (long long i = grp; i < cnt; i += G) {\n"
       << "   const long long w = first + i, b = w >> a.g.n_out;\n"
@@ -1385,7 +1395,8 @@ size_t jit_forward_smem(const Pass &p, int precision) { return fwd_smem(p, preci
 
 size_t jit_backward_smem(const Pass &p, int precision, int n_hams) {
     const size_t buf = (size_t(1) << p.K) * elem_bytes(precision) * (1 + n_hams);
-    return size_t(bwd_buffers(p, precision, n_hams)) * buf + bwd_fixed_smem(p, precision, n_hams);
+    const int scratch = bwd_scratch(p, precision, n_hams);
+    return size_t(bwd_buffers(p, precision, n_hams, scratch)) * buf + bwd_fixed_smem(p, precision, n_hams, scratch);
 }
 
 namespace {

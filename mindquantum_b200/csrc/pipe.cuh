@@ -161,8 +161,8 @@ __device__ __forceinline__ void pass_phase(V *ph, const V *mtab, const JitMtab *
     if (tid == 0u) *ph = reg::cval<V>(p.x, p.y);
 }
 
-// Gradient rows of a warp: 512 bytes of shared scratch at `scr` hold 4 rows of 32 float partials (2 of
-// double).  row_put stores this lane's partial of row k; rows_flush_as adds the n rows over the lanes (in
+// Gradient rows of a warp: shared scratch at `scr` holds N = 4 or 8 rows of 32 float partials, or 2 of double.
+// row_put stores this lane's partial of row k; rows_flush_as adds the n rows over the lanes (in
 // the partials' precision) and the sums to acc[0..n) in FP64.  The accesses are volatile asm without a
 // memory clobber: they keep their order among themselves, and the compiler may move the gates' own
 // shared-memory reads across them.
@@ -172,15 +172,26 @@ __device__ __forceinline__ void row_put(unsigned scr, int k, int lane, float x) 
 __device__ __forceinline__ void row_put(unsigned scr, int k, int lane, double x) {
     asm volatile("st.shared.f64 [%0], %1;" ::"r"(scr + unsigned(k * 32 + lane) * 8u), "d"(x));
 }
-__device__ __forceinline__ void rows_sum(unsigned scr, int lane, float &s, int &row, bool &first) {
+__device__ __forceinline__ float four(unsigned at) {
     float x, y, z, w;
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x), "=f"(y), "=f"(z), "=f"(w) : "r"(scr + unsigned(lane) * 16u));
-    s = (x + y) + (z + w);
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    row = lane >> 3;
-    first = (lane & 7) == 0;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x), "=f"(y), "=f"(z), "=f"(w) : "r"(at));
+    return (x + y) + (z + w);
 }
+template <int N>
+__device__ __forceinline__ void rows_sum(unsigned scr, int lane, float &s, int &row, bool &first) {
+    constexpr int LR = 32 / N;   // lanes per row
+    row = lane / LR;
+    if (N == 8) {   // two 16-byte chunks per lane, in turned order on odd rows (distinct banks in a quarter-warp)
+        const unsigned at = scr + unsigned(row * 128 + (lane & 3) * 16), turn = (row & 1) ? 64u : 0u;
+        s = four(at + turn) + four(at + (64u ^ turn));
+    } else {
+        s = four(scr + unsigned(lane) * 16u);
+    }
+#pragma unroll
+    for (int o = LR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    first = lane % LR == 0;
+}
+template <int N>
 __device__ __forceinline__ void rows_sum(unsigned scr, int lane, double &s, int &row, bool &first) {
     double x, y;
     asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(x), "=d"(y) : "r"(scr + unsigned(lane) * 16u));
@@ -191,13 +202,13 @@ __device__ __forceinline__ void rows_sum(unsigned scr, int lane, double &s, int 
     first = (lane & 15) == 0;
 }
 __device__ __forceinline__ void warp_order() { asm volatile("bar.warp.sync 0xffffffff;"); }
-template <typename R>
+template <typename R, int N>
 __device__ __forceinline__ void rows_flush_as(unsigned scr, double *acc, int n, int lane) {
     R s;
     int row;
     bool first;
     warp_order();
-    rows_sum(scr, lane, s, row, first);
+    rows_sum<N>(scr, lane, s, row, first);
     warp_order();
     if (first && row < n) acc[row] += double(s);
 }
