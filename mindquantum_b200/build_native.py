@@ -19,10 +19,10 @@ LIB = os.path.join(HERE, 'libmqb200.so')
 FUSED = ['fused_fwd_c64.cu', 'fused_fwd_c128.cu', 'fused_bwd_c64.cu', 'fused_bwd_c128.cu']
 SOURCES = ['kernels.cu', 'small.cu', *FUSED, 'capi.cpp', 'scheduler.cpp', 'noalloc.cu', 'jit.cpp']
 HEADERS = ['kernels.cuh', 'small.h', 'mqb_internal.h', 'mqb_gate_ids.h', 'fused_impl.cuh', 'regops.cuh', 'regmath.cuh',
-           'tile.cuh', 'jit_abi.h', 'jit.h', 'pipe.cuh', 'phasemath.cuh']
+           'tile.cuh', 'jit_abi.h', 'jit.h', 'pipe.cuh']
 # headers compiled again at run time by NVRTC for the generated pass kernels (embedded as text)
 JIT_HEADERS = [('kJitRegmath', 'regmath.cuh'), ('kJitTile', 'tile.cuh'), ('kJitAbi', 'jit_abi.h'),
-               ('kJitPipe', 'pipe.cuh'), ('kJitPhase', 'phasemath.cuh')]
+               ('kJitPipe', 'pipe.cuh')]
 # NVRTC from the CUDA toolkit the library is built with (found again at run time through the rpath)
 CUDA_LIB = '/usr/local/cuda/lib64'
 NVRTC_LIBS = [f'-L{CUDA_LIB}', '-lnvrtc', '-Xlinker', f'-rpath={CUDA_LIB}']

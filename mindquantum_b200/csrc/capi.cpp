@@ -251,7 +251,7 @@ JitBlock::~JitBlock() { t_jit_blocked = prev_; }
 
 static std::vector<JitMtab> jit_mtab(const std::vector<StageOp> &v) {
     std::vector<JitMtab> o(v.size());
-    for (size_t i = 0; i < v.size(); ++i) o[i] = JitMtab{v[i].moff, v[i].mcount, (long long)v[i].msrc, v[i].msrc_ps, v[i].phase & ~kPhaseUnitary};
+    for (size_t i = 0; i < v.size(); ++i) o[i] = JitMtab{v[i].moff, v[i].mcount, (long long)v[i].msrc, v[i].msrc_ps, v[i].norm};
     return o;
 }
 
@@ -458,7 +458,6 @@ static void run_matgen(const mqb_program &p, const double *params, int64_t param
     m.batch = batch;
     m.mats = mats;
     m.mats_stride = p.per_sample;
-    m.ratios = p.use_jit();
     TimeScope ts(TK_MATGEN, st);
     ck(launch_matgen<R>(m, st), "matgen");
 }

@@ -32,12 +32,11 @@
 
 namespace mqb {
 
-// Header texts for NVRTC, embedded at build time from regmath.cuh, tile.cuh, jit_abi.h, pipe.cuh and phasemath.cuh.
+// Header texts for NVRTC, embedded at build time from regmath.cuh, tile.cuh, jit_abi.h and pipe.cuh.
 extern const char *const kJitRegmath;
 extern const char *const kJitTile;
 extern const char *const kJitAbi;
 extern const char *const kJitPipe;
-extern const char *const kJitPhase;
 
 namespace {
 
@@ -323,13 +322,21 @@ void emit_backward_op(std::ostringstream &o, const StageOp &so, int NH, int gid,
 // ------------------------------------------------------------------ diagonal gates of known unitaries
 // Consecutive diagonal gates of a stage commute, and most of their work can be taken out of the
 // per-amplitude path:
-//   * A pair (d0, d1) on a register bit is d0 times (1, r) with r = d1 / d0 (kept in the matrix table): only the amplitudes with
-//     the bit set are multiplied, a run of k such gates by a table of 2^k - 1 products (a ZZ pair the same way,
-//     by the parity of its two bits).
-//   * What is the same for all of a thread's amplitudes, a gate whose targets are off the registers
-//     or a taken-out d0, commutes with everything else the stage does to the registers: such factors
-//     collect in one scalar `sc` per thread, applied once at the end of the stage.  Factors that are the
-//     same for every thread (d0 of an uncontrolled gate) wait for the end of the pass (`ph`, made with the table).
+//   * The factors of gates that are the same for every thread (targets and controls on register bits) come from a table
+//     in shared memory, an entry per value of the bits that the run depends on, made once per sample
+//     (pipe::load_runs): a run costs one product per amplitude.
+//   * Gates on register bits whose factor depends on the thread (a control or the other target of a ZZ pair off the
+//     registers) multiply a table that the thread makes.
+//   * What is the same for all of a thread's amplitudes, a gate whose targets are off the registers, commutes
+//     with everything else the stage does to the registers: such factors collect in one scalar `sc` per
+//     thread, applied at the end of the stage.
+// A pair (d0, d1) enters with both entries, as rounded, and the products are taken in FP64.  The entries
+// of a rotation are conjugates, so that their rounding scales the state as a whole, which the factor of
+// pipe::pass_norm takes out.  Taking d0 out and keeping the ratio d1 / d0 halves the products, but its rounded modulus
+// differs from one on half of the amplitudes only, and so do products rounded to complex64: that moved the 26-qubit,
+// 12-layer expectation (values of 0.005 to 0.1, ten parameter sets) by 1.4e-7 and 7.9e-8 rms, the rounding of
+// the matrices by 5.1e-8, and by 2.3e-8 without the norm.  Here it is off by 4.1e-8, most of which the first two passes' arithmetic
+// adds on the few amplitudes that are not zero yet.  The price on that gradient (batch 2): 49.6 -> 53.5 ms.
 //   * In the adjoint, the sum S of Im(conj(lambda) psi) over a thread's amplitudes does not change under
 //     what the stage does to both states, so it is computed once per stage; a gate's gradient is then
 //     w0 S + (w1 - w0) SB with SB the sum over the amplitudes its bit selects, and a gate off
@@ -338,7 +345,7 @@ void emit_backward_op(std::ostringstream &o, const StageOp &so, int NH, int gid,
 
 // State of the stage that is being written.
 struct StageCtx {
-    bool sc = false;   // `sc` carries a factor
+    bool sc = false;   // `sc` (FP64) carries a factor
     bool S = false;    // `S` holds the thread's sums
     int id = 0;
 };
@@ -347,16 +354,13 @@ bool diag_op(const StageOp &so) { return so.kind == SK_DIAG1 || so.kind == SK_DI
 
 // Gates a run may hold: diagonal, unitary, and (adjoint) no gradient or a generator-form one.
 bool phase_op(const StageOp &so, int gid, bool adj) {
-    if (!diag_op(so) || !(so.phase & kPhaseUnitary)) return false;
+    if (!diag_op(so) || !so.unitary) return false;
     const int G = so.n_angles ? so.grad_mask : 0;
     return !adj || G == 0 || (G == 1 && !phase_weights(gid).empty());
 }
 
-// Whether the op leaves a factor for the end of its pass (pipe::pass_phase).
-bool leaves_factor(const StageOp &so) { return (so.phase & kPhaseKind) == kPhaseUniform || so.phase >> kPhaseNormShift; }
-
 // Whether the thread's S survives the op: unitary on its registers.
-bool keeps_sums(const StageOp &so) { return so.phase & kPhaseUnitary; }
+bool keeps_sums(const StageOp &so) { return so.unitary != 0; }
 
 enum PhaseShape { PH_OFF, PH_BIT, PH_PARITY, PH_OTHER };
 PhaseShape phase_shape(const StageOp &so, int gid) {
@@ -369,13 +373,81 @@ PhaseShape phase_shape(const StageOp &so, int gid) {
 }
 int phase_bit(const StageOp &so) { return so.dsrc[0] == 0 ? so.dval[0] : so.dval[1]; }
 
+// Factor tables of a pass's runs in shared memory.  Complex64 alone: complex128 products lose nothing that matters.
+struct RunTables {
+    // 16 runs of four bits; a pass of more makes the rest of its runs' factors in each thread
+    static constexpr size_t kMaxEntries = 256;
+    struct Gate {
+        int moff, p0, p1;
+        unsigned ctrl;
+    };
+    struct Entry {
+        size_t first;
+        int n, idx;
+    };
+    std::vector<Gate> gates;
+    std::vector<Entry> entries;
+
+    static bool takes(const StageOp &so, int gid) {
+        if (!on_expr(so).empty() || gid == GID_GP) return false;
+        return so.dsrc[0] == 0 && (so.kind != SK_DIAG2 || so.dsrc[1] == 0);
+    }
+    // The first entry of the table of `run` over the register bits `bits` (set here); -1: it gets none.
+    int add(const std::vector<const StageOp *> &run, std::vector<int> &bits) {
+        if (run.size() < 2 || run.size() > 255) return -1;
+        unsigned used = 0;
+        for (const StageOp *so : run) {
+            used |= so->rctrl | 1u << so->dval[0];
+            if (so->kind == SK_DIAG2) used |= 1u << so->dval[1];
+        }
+        for (int P = 0; P < kMaxRegBits; ++P)
+            if (used >> P & 1) bits.push_back(P);
+        const size_t at = entries.size(), n = size_t(1) << bits.size();
+        if (at + n > kMaxEntries || gates.size() + run.size() > 65535) return -1;
+        auto place = [&](int P) { return int(std::find(bits.begin(), bits.end(), P) - bits.begin()); };
+        for (size_t idx = 0; idx < n; ++idx) entries.push_back({gates.size(), int(run.size()), int(idx)});
+        for (const StageOp *so : run) {
+            unsigned ctrl = 0;
+            for (size_t k = 0; k < bits.size(); ++k)
+                if (so->rctrl >> bits[k] & 1) ctrl |= 1u << k;
+            gates.push_back({so->moff, place(so->dval[0]), so->kind == SK_DIAG2 ? place(so->dval[1]) : -1, ctrl});
+        }
+        return int(at);
+    }
+    void declare(std::ostringstream &o) const {
+        if (entries.empty()) return;
+        o << "__device__ const pipe::RunGate run_gates[" << gates.size() << "] = {";
+        for (const Gate &g : gates) o << "{" << g.moff << ", " << g.p0 << ", " << g.p1 << ", " << g.ctrl << "}, ";
+        o << "};\n__device__ const pipe::RunEntry run_entries[" << entries.size() << "] = {";
+        for (const Entry &e : entries) o << "{" << e.first << ", " << e.n << ", " << e.idx << "}, ";
+        o << "};\n";
+    }
+};
+
+// The ops of a stage in execution order: runs of diagonal gates to `run`, others to `single`.
+template <typename F, typename G>
+void walk_stage(const StageDesc &sd, const StageOp *sops, const std::vector<DevOp> &ops, bool adj, F run, G single) {
+    const int n = sd.op_end - sd.op_begin;
+    auto at = [&](int i) -> const StageOp & { return sops[adj ? sd.op_end - 1 - i : sd.op_begin + i]; };
+    for (int i = 0; i < n;) {
+        std::vector<const StageOp *> r;
+        std::vector<int> gids;
+        for (; i < n && phase_op(at(i), ops[at(i).op].gate_id, adj); ++i) {
+            r.push_back(&at(i));
+            gids.push_back(ops[at(i).op].gate_id);
+        }
+        if (!r.empty()) run(r, gids);
+        else single(at(i++));
+    }
+}
+
 void emit_phase_run(std::ostringstream &o, const std::vector<const StageOp *> &run, const std::vector<int> &gids, int RB,
-                    Rows *rows, StageCtx &ctx) {
+                    Rows *rows, RunTables *tables, StageCtx &ctx) {
     const bool adj = rows != nullptr;
     const int id = ctx.id++;
     const std::string u = "_" + std::to_string(id);
     auto ent = [&](int M, const std::string &idx) {
-        const std::string e = "mt[" + std::to_string(M) + " + " + idx + "]";
+        const std::string e = "pipe::wide(mt[" + std::to_string(M) + " + " + idx + "])";
         return adj ? "cconj(" + e + ")" : e;
     };
     auto grads = [](const StageOp &so) { return so.n_angles ? so.grad_mask : 0; };
@@ -501,14 +573,47 @@ void emit_phase_run(std::ostringstream &o, const std::vector<const StageOp *> &r
         }
     }
 
-    // the factor table over the register bits that the gates depend on
+    // the run's table in shared memory
+    std::vector<size_t> own;   // gates whose factors the thread makes
+    {
+        std::vector<const StageOp *> same;
+        std::vector<size_t> rest;
+        std::vector<int> bits;
+        for (size_t k = 0; k < run.size(); ++k) {
+            if (tables && RunTables::takes(*run[k], gids[k])) same.push_back(run[k]);
+            else rest.push_back(k);
+            own.push_back(k);
+        }
+        const int at = tables ? tables->add(same, bits) : -1;
+        if (at >= 0) {
+            own = rest;
+            for (int idx = 0; idx < 1 << bits.size(); ++idx) {
+                o << "    {\n     const auto d = runs[" << at + idx << "];\n";
+                for (int j = 0; j < (1 << RB); ++j) {
+                    bool in = true;
+                    for (size_t k = 0; k < bits.size(); ++k) in = in && ((j >> bits[k] & 1) == (idx >> k & 1));
+                    if (!in) continue;
+                    o << "     v[" << j << "] = pipe::times(v[" << j << "], d);";
+                    if (adj) o << " for (int h = 0; h < NH; ++h) l[h][" << j << "] = pipe::times(l[h][" << j << "], d);";
+                    o << "\n";
+                }
+                o << "    }\n";
+            }
+        }
+    }
+    if (own.empty()) return;
+
+    // the thread's table over the register bits that the other gates depend on, and its scalar
     std::vector<int> tb;
     auto use = [&](int P) {
         if (std::find(tb.begin(), tb.end(), P) == tb.end()) tb.push_back(P);
     };
-    for (size_t k = 0; k < run.size(); ++k) {
+    bool mirrored = true;   // the table's entries at idx and ~idx are conjugates: rotations by Z and ZZ alone
+    for (size_t k : own) {
         const StageOp &so = *run[k];
-        if (phase_shape(so, gids[k]) == PH_OFF) continue;
+        const PhaseShape sh = phase_shape(so, gids[k]);
+        if (sh == PH_OFF) continue;
+        mirrored = mirrored && sh == PH_BIT && (gids[k] == GID_RZ || gids[k] == GID_RZZ);
         for (int t = 0; t < (so.kind == SK_DIAG2 ? 2 : 1); ++t)
             if (so.dsrc[t] == 0) use(so.dval[t]);
         for (int P = 0; P < RB; ++P)
@@ -524,65 +629,50 @@ void emit_phase_run(std::ostringstream &o, const std::vector<const StageOp *> &r
             return;
         }
         const std::string name = "t" + u + "_" + std::to_string(n_tmp++);
-        o << "    const V " << name << " = cmul(" << t << ", " << f << ");\n";
+        o << "    const W " << name << " = cmul(" << t << ", " << f << ");\n";
         t = name;
     };
     auto idx_bit = [&](int idx, int P) { return (idx >> (std::find(tb.begin(), tb.end(), P) - tb.begin())) & 1; };
-    auto scale_by = [&](const std::string &f) {
-        o << "    sc = " << (ctx.sc ? "cmul(sc, " + f + ")" : f) << ";\n";
-        ctx.sc = true;
-    };
-    std::map<int, std::string> ratio;   // register bit -> product of its gates' ratios
-    for (size_t k = 0; k < run.size(); ++k) {
+    std::map<int, std::pair<std::string, std::string>> pairs;   // register bit -> products of its gates' entries
+    for (size_t k : own) {
         const StageOp &so = *run[k];
         const std::string on = on_expr(so);
-        auto sel = [&](const std::string &f) { return on.empty() ? f : "((" + on + ") ? " + f + " : cval<V>(1, 0))"; };
+        auto sel = [&](const std::string &f) { return on.empty() ? f : "((" + on + ") ? " + f + " : cval<W>(1, 0))"; };
         const PhaseShape sh = phase_shape(so, gids[k]);
-        const bool uniform = (so.phase & kPhaseKind) == kPhaseUniform;   // d0 waits for the end of the pass, the table holds r
-        if (sh == PH_OFF && !uniform) scale_by(sel(ent(so.moff, off_index(so, gids[k]))));
-        if (sh != PH_BIT) continue;
-        const std::string r = "r" + u + "_" + std::to_string(k);
-        if (uniform) {
-            o << "    const V " << r << " = " << ent(so.moff, "1") << ";\n";
-        } else if (so.kind == SK_DIAG1) {
-            o << "    const V " << r << " = " << sel(ent(so.moff, "1")) << ";\n";
-            scale_by(sel(ent(so.moff, "0")));
-        } else {   // entries (a, b, b, a), b / a at 1: the other target's bit swaps a and b
-            const std::string b = "(" + off_bit_expr(so.dsrc[so.dsrc[0] == 0 ? 1 : 0], so.dval[so.dsrc[0] == 0 ? 1 : 0]) + ")";
-            o << "    const V " << r << "a = " << ent(so.moff, "1") << ", " << r << " = "
-              << sel("(" + b + " ? cconj(" + r + "a) : " + r + "a)") << ";\n";
-            scale_by(sel("(" + b + " ? " + ent(so.moff, "2") + " : " + ent(so.moff, "0") + ")"));
+        if (sh == PH_OFF) {
+            const std::string f = sel(ent(so.moff, off_index(so, gids[k])));
+            o << "    sc = " << (ctx.sc ? "cmul(sc, " + f + ")" : f) << ";\n";
+            ctx.sc = true;
         }
-        times(ratio[phase_bit(so)], r);
+        if (sh != PH_BIT) continue;
+        auto &p = pairs[phase_bit(so)];
+        const auto ix = so.kind == SK_DIAG1 ? std::make_pair(std::string("0"), std::string("1")) : pair_index(so);
+        if (gids[k] != GID_PS) times(p.first, sel(ent(so.moff, ix.first)));   // (a phase shift's first entry is 1)
+        if (!mirrored) times(p.second, sel(ent(so.moff, ix.second)));
     }
-    // products over the bits' ratios, lowest bit first
-    for (int idx = 1; idx < nt; ++idx) {
-        int top = -1;
-        for (size_t k = 0; k < tb.size(); ++k)
-            if ((idx >> k & 1) && ratio.count(tb[k])) top = int(k);
-        if (top < 0) continue;
-        T[size_t(idx)] = T[size_t(idx & ~(1 << top))];
-        // (without the bits above `top`, which carry no ratio, the entry is already there)
-        const int core = idx & ((2 << top) - 1);
-        if (core != idx) T[size_t(idx)] = T[size_t(core)];
-        else times(T[size_t(idx)], ratio[tb[size_t(top)]]);
+    if (tb.empty()) return;
+    // products over the bits' pairs, lowest bit first; of a mirrored table the half whose top bit is clear
+    if (mirrored) T[0] = pairs[tb.back()].first;
+    for (size_t k = 0; k + (mirrored ? 1 : 0) < tb.size(); ++k) {
+        const auto it = pairs.find(tb[k]);
+        for (size_t idx = 0; idx < size_t(1) << k; ++idx) {
+            const size_t up = idx | size_t(1) << k;
+            T[up] = T[idx];
+            if (it == pairs.end()) continue;
+            times(T[up], mirrored ? "cconj(" + it->second.first + ")" : it->second.second);
+            if (!it->second.first.empty()) times(T[idx], it->second.first);
+        }
     }
-    for (size_t k = 0; k < run.size(); ++k) {
+    if (mirrored)
+        for (int idx = 0; idx < nt / 2; ++idx) T[size_t(nt - 1 - idx)] = "cconj(" + T[size_t(idx)] + ")";
+    for (size_t k : own) {
         const StageOp &so = *run[k];
         const std::string on = on_expr(so);
-        auto sel = [&](const std::string &f) { return on.empty() ? f : "((" + on + ") ? " + f + " : cval<V>(1, 0))"; };
+        auto sel = [&](const std::string &f) { return on.empty() ? f : "((" + on + ") ? " + f + " : cval<W>(1, 0))"; };
         const PhaseShape sh = phase_shape(so, gids[k]);
         if (sh == PH_PARITY) {
-            const bool uniform = (so.phase & kPhaseKind) == kPhaseUniform;
-            const std::string r = "r" + u + "_" + std::to_string(k);
-            if (uniform) {
-                o << "    const V " << r << " = " << ent(so.moff, "1") << ";\n";
-            } else {
-                o << "    const V " << r << " = " << sel(ent(so.moff, "1")) << ";\n";
-                scale_by(sel(ent(so.moff, "0")));
-            }
             for (int idx = 0; idx < nt; ++idx)
-                if (idx_bit(idx, so.dval[0]) ^ idx_bit(idx, so.dval[1])) times(T[size_t(idx)], r);
+                times(T[size_t(idx)], sel(ent(so.moff, (idx_bit(idx, so.dval[0]) ^ idx_bit(idx, so.dval[1])) ? "1" : "0")));
         } else if (sh == PH_OTHER) {
             for (int idx = 0; idx < nt; ++idx) {
                 bool set = true;
@@ -601,7 +691,7 @@ void emit_phase_run(std::ostringstream &o, const std::vector<const StageOp *> &r
     }
     for (int idx = 0; idx < nt; ++idx) {
         if (T[size_t(idx)].empty()) continue;
-        o << "    {\n     const V d = " << T[size_t(idx)] << ";\n";
+        o << "    {\n     const W dw = " << T[size_t(idx)] << ";\n     const V d = cval<V>(dw.x, dw.y);\n";
         for (int j = 0; j < (1 << RB); ++j) {
             bool in = true;
             for (size_t k = 0; k < tb.size(); ++k) in = in && ((j >> tb[k] & 1) == (idx >> k & 1));
@@ -614,17 +704,21 @@ void emit_phase_run(std::ostringstream &o, const std::vector<const StageOp *> &r
     }
 }
 
-// The factors that a stage's diagonal gates left for its end (and, in the last stage of a pass, the pass's).
-void emit_stage_phase(std::ostringstream &o, int RB, bool adj, const StageCtx &ctx, bool last, bool pass_phase) {
-    if (!ctx.sc && !pass_phase) return;
-    const std::string ph = adj ? "cconj(*ph)" : "*ph";
-    o << "    {\n     const V d = " << (ctx.sc ? (pass_phase ? "cmul(sc, " + ph + ")" : "sc") : ph) << ";\n";
+// The factor that a stage's diagonal gates left for its end and, in the last stage, the pass's norm.
+void emit_stage_phase(std::ostringstream &o, int RB, bool adj, const StageCtx &ctx, bool last, bool norm) {
+    norm = norm && last;
+    if (!ctx.sc && !norm) return;
+    if (ctx.sc) o << "    {\n     const double q = " << (norm ? "*ph" : "1") << ";\n     const V d = cval<V>(sc.x * q, sc.y * q);\n";
+    else o << "    {\n     const R q = R(*ph - 1.0);   // (1 + q rounded would leave 3e-8 per pass)\n";
+    auto scale = [&](const std::string &x) {
+        return ctx.sc ? x + " = cmul(" + x + ", d);" : x + " = cval<V>(fma(" + x + ".x, q, " + x + ".x), fma(" + x + ".y, q, " + x + ".y));";
+    };
     if (adj && last) o << "     if (a.psi_dst) {\n";   // psi leaves the last stage only where it is stored
-    for (int j = 0; j < (1 << RB); ++j) o << "     v[" << j << "] = cmul(v[" << j << "], d);\n";
+    for (int j = 0; j < (1 << RB); ++j) o << "     " << scale("v[" + std::to_string(j) + "]") << "\n";
     if (adj && last) o << "     }\n";
     if (adj)
         for (int j = 0; j < (1 << RB); ++j)
-            o << "     for (int h = 0; h < NH; ++h) l[h][" << j << "] = cmul(l[h][" << j << "], d);\n";
+            o << "     for (int h = 0; h < NH; ++h) { " << scale("l[h][" + std::to_string(j) + "]") << " }\n";
     o << "    }\n";
 }
 
@@ -825,10 +919,14 @@ int fwd_buffers(const Pass &p, int precision) {
     return std::max(fwd_groups(p, precision), env_int("MQB_PIPE_FWD_BUFFERS", precision == MQB_PREC_C64 ? 2 : 3, 1, 8));
 }
 
+// The ring's mbarriers and tickets, and the pass norm of each group.
+constexpr size_t kRingBytes = 8 * 16 + 8 * 16;
+constexpr size_t kSplitBytes = 16;   // sizeof(pipe::Split)
+
 size_t fwd_smem(const Pass &p, int precision) {
     const size_t eb = elem_bytes(precision);
     return size_t(fwd_buffers(p, precision)) * ((size_t(1) << p.K) * eb) +
-           size_t(fwd_groups(p, precision)) * a16(size_t(p.f_mtab_entries) * eb) + 8 * 16 + 16 * size_t(eb);
+           size_t(fwd_groups(p, precision)) * (a16(size_t(p.f_mtab_entries) * eb) + size_t(p.f_run_entries) * kSplitBytes) + kRingBytes;
 }
 
 int bwd_groups(const Pass &p) {
@@ -836,38 +934,43 @@ int bwd_groups(const Pass &p) {
     return std::min(max_groups(nt), env_int("MQB_PIPE_BWD_GROUPS", 2, 1, 15));
 }
 
-size_t bwd_fixed_smem(const Pass &p, int precision, int n_hams, int scratch) {
+size_t bwd_fixed_smem(const Pass &p, int precision, int n_hams, int scratch, int runs) {
     const size_t eb = elem_bytes(precision);
     const int nw = (1 << (p.K - p.reg_bits)) / 32;
     return size_t(bwd_groups(p)) *
                (a16(size_t(p.mtab_entries) * eb) + a16(size_t(nw) * std::max(1, p.n_slots) * n_hams * sizeof(double)) +
-                size_t(nw) * size_t(scratch)) +
-           8 * 16 + 16 * size_t(eb);
+                size_t(nw) * size_t(scratch) + a16(size_t(runs) * eb)) +
+           kRingBytes;
 }
 
 // Buffers of the adjoint ring: G + 1 where they fit in 227 KB, else as many as fit (at least G); 0: fewer than
 // G fit.
-int bwd_buffers(const Pass &p, int precision, int n_hams, int scratch) {
+int bwd_buffers(const Pass &p, int precision, int n_hams, int scratch, int runs) {
     const size_t buf = (size_t(1) << p.K) * elem_bytes(precision) * (1 + n_hams);
-    const size_t fixed = bwd_fixed_smem(p, precision, n_hams, scratch);
+    const size_t fixed = bwd_fixed_smem(p, precision, n_hams, scratch, runs);
     const int G = bwd_groups(p);
     int nb = env_int("MQB_PIPE_BWD_BUFFERS", G + 1, 1, 8);
     while (nb > G && nb * buf + fixed > size_t(227) << 10) --nb;
     return nb * buf + fixed > size_t(227) << 10 ? 0 : nb;
 }
 
-// Bytes of gradient-row scratch per warp: four rows (two in complex128), or eight complex64 rows where they
-// cost the ring no buffer.
-int bwd_scratch(const Pass &p, int precision, int n_hams) {
-    const int nb = bwd_buffers(p, precision, n_hams, 512);
-    if (nb == 0) throw std::runtime_error("generated adjoint pass: the tile ring does not fit in shared memory");
-    return precision == MQB_PREC_C64 && bwd_buffers(p, precision, n_hams, 1024) == nb ? 1024 : 512;
+// Bytes of gradient-row scratch per warp, entries of the runs' tables and ring buffers of an adjoint kernel.  Scratch: four
+// rows (two in complex128), or eight complex64 rows; the tables and the eight rows where they cost the ring no buffer.
+struct BwdShape {
+    int scratch, runs, buffers;
+};
+BwdShape bwd_shape(const Pass &p, int precision, int n_hams) {
+    BwdShape b{512, 0, bwd_buffers(p, precision, n_hams, 512, 0)};
+    if (b.buffers == 0) throw std::runtime_error("generated adjoint pass: the tile ring does not fit in shared memory");
+    if (bwd_buffers(p, precision, n_hams, 512, p.run_entries) == b.buffers) b.runs = p.run_entries;
+    if (precision == MQB_PREC_C64 && bwd_buffers(p, precision, n_hams, 1024, b.runs) == b.buffers) b.scratch = 1024;
+    return b;
 }
 
 void emit_header(std::ostringstream &o, int precision) {
     o << "#include \"regmath.cuh\"\n#include \"tile.cuh\"\n#include \"pipe.cuh\"\n"
       << "using namespace mqb;\nusing namespace mqb::reg;\n"
-      << "typedef " << vname(precision) << " V;\ntypedef " << rname(precision) << " R;\n";
+      << "typedef " << vname(precision) << " V;\ntypedef " << rname(precision) << " R;\ntypedef double2 W;\n";
 }
 
 uint32_t reg_local(const StageDesc &sd, int RB, int j) {
@@ -986,6 +1089,13 @@ void emit_ring_exit(std::ostringstream &o) {
       << "   pipe::bulk_wait_all();\n  }\n";
 }
 
+// What a group makes of a new sample's matrix table: the pass norm and the runs' tables.
+void emit_load_derived(std::ostringstream &o, bool norm, int run_entries) {
+    if (norm) o << "    pipe::pass_norm(ph, mt, a.mt, a.n_mt, tid);\n";
+    if (run_entries) o << "    pipe::load_runs(runs, mt, run_gates, run_entries, " << run_entries << ", tid, NT);\n";
+    if (norm || run_entries) o << "    pipe::consumers_sync(BAR, NT);\n";
+}
+
 std::string forward_source(const Schedule &s, const Pass &p, int precision, const std::vector<DevOp> &ops) {
     const int RB = p.f_reg_bits, K = p.K, TB = K - RB;
     const PassPlan pl = pass_plan(p.qbits, precision);
@@ -993,13 +1103,13 @@ std::string forward_source(const Schedule &s, const Pass &p, int precision, cons
     std::vector<const StageDesc *> ex;
     for (int si = 0; si < p.f_n_stages; ++si) ex.push_back(&s.f_stages[p.f_stage_begin + si]);
     const LayPlan lp = plan_layouts(pl, ex, TB);
-    bool pass_phase = false;
-    for (int k = 0; k < p.f_n_sops; ++k) pass_phase = pass_phase || leaves_factor(s.f_stage_ops[p.f_sop_begin + k]);
     // blocks per SM that the shared-memory ring allows, up to 24 warps: the register budget is sized for them
     const size_t fit = (size_t(220) << 10) / fwd_smem(p, precision), most = size_t(768) / size_t(G << TB);
     const int min_blocks = int(std::max<size_t>(1, std::min(most, fit)));
+    const StageOp *sops = s.f_stage_ops.data() + p.f_sop_begin;
+    const bool norm = std::any_of(sops, sops + p.f_n_sops, [](const StageOp &so) { return so.norm != 0; });
+    RunTables tables;
     std::ostringstream o;
-    emit_header(o, precision);
     o << "extern \"C\" __global__ void __launch_bounds__(" << G * (1 << TB) << ", " << min_blocks
       << ") mqb_fwd_pass(const JitFwdArgs<V> a, "
       << "const __grid_constant__ pipe::TMap m_src, const __grid_constant__ pipe::TMap m_dst) {\n"
@@ -1010,7 +1120,6 @@ std::string forward_source(const Schedule &s, const Pass &p, int precision, cons
       << "  const tile::u64 mtb = tile::align16(tile::u64(a.mtab_entries) * sizeof(V));\n"
       << "  pipe::u64 *full = reinterpret_cast<pipe::u64 *>(smem + NB * BUFB + G * mtb);\n"
       << "  volatile long long *ticket = reinterpret_cast<volatile long long *>(full + NB);\n"
-      << "  V *ph = reinterpret_cast<V *>(full + 16) + int(threadIdx.x) / NT;   // factor left for the end of the pass\n"
       << "  if (threadIdx.x == 0) {\n   for (int k = 0; k < NB; ++k) {\n    pipe::mbar_init(full + k, 1);\n    ticket[k] = -1;\n   }\n"
       << "   pipe::fence_mbar_init();\n  }\n  __syncthreads();\n"
       << "  const long long n_tiles = 1ll << a.g.n_out, total = a.batch * n_tiles;\n"
@@ -1020,6 +1129,8 @@ std::string forward_source(const Schedule &s, const Pass &p, int precision, cons
                        "   pipe::load_tile(&m_src, a.tg, (bs << n) | tb, buf, full + sb);\n",
                        true);
     o << "  V *mt = reinterpret_cast<V *>(smem + NB * BUFB + grp * mtb);\n"
+      << "  double *ph = reinterpret_cast<double *>(full + 16) + grp;\n"
+      << "  pipe::Split *runs = reinterpret_cast<pipe::Split *>(full + 32) + grp * " << p.f_run_entries << ";\n"
       << "  long long cached_b = -1;\n"
       << "  for (long long i = grp; i < cnt; i += G) {\n"
       << "   const long long w = first + i, b = w >> a.g.n_out;\n"
@@ -1028,8 +1139,9 @@ std::string forward_source(const Schedule &s, const Pass &p, int precision, cons
       << "   V *tl = reinterpret_cast<V *>(smem + sb * BUFB);\n"
       << "   if (b != cached_b) {\n    pipe::consumers_sync(BAR, NT);\n"
       << "    pipe::load_mtab(mt, a.mt, a.n_mt, a.mats + b * a.mats_stride, a.cpool, tid, NT);\n"
-      << "    cached_b = b;\n    pipe::consumers_sync(BAR, NT);\n"
-      << (pass_phase ? "    pipe::pass_phase(ph, mt, a.mt, a.n_mt, tid);\n    pipe::consumers_sync(BAR, NT);\n" : "") << "   }\n";
+      << "    cached_b = b;\n    pipe::consumers_sync(BAR, NT);\n";
+    emit_load_derived(o, norm, p.f_run_entries);
+    o << "   }\n";
     emit_ring_wait(o);
     if (lp.relayout_in) {
         o << "   if (!zero) {\n    V *tbase = tl;\n";
@@ -1041,20 +1153,14 @@ std::string forward_source(const Schedule &s, const Pass &p, int precision, cons
         const bool last = si + 1 == ex.size();
         emit_stage_load(o, pl, sd, RB, TB, 0, lp.in[si], si == 0);
         StageCtx ctx;
-        o << "    V sc = cval<V>(1, 0);\n";
-        for (int k = sd.op_begin; k < sd.op_end;) {
-            std::vector<const StageOp *> run;
-            std::vector<int> gids;
-            for (; k < sd.op_end; ++k) {
-                const StageOp &so = s.f_stage_ops[p.f_sop_begin + k];
-                if (!phase_op(so, ops[so.op].gate_id, false)) break;
-                run.push_back(&so);
-                gids.push_back(ops[so.op].gate_id);
-            }
-            if (!run.empty()) emit_phase_run(o, run, gids, RB, nullptr, ctx);
-            else emit_forward_op(o, s.f_stage_ops[p.f_sop_begin + k++]);
-        }
-        emit_stage_phase(o, RB, false, ctx, last, last && pass_phase);
+        o << "    W sc = cval<W>(1, 0);\n";
+        walk_stage(
+            sd, sops, ops, false,
+            [&](const std::vector<const StageOp *> &run, const std::vector<int> &gids) {
+                emit_phase_run(o, run, gids, RB, nullptr, p.f_run_entries ? &tables : nullptr, ctx);
+            },
+            [&](const StageOp &so) { emit_forward_op(o, so); });
+        emit_stage_phase(o, RB, false, ctx, last, norm);
         if (last)   // the FP64 norm check of the output, when the launch asks for it
             o << "    if (a.norm) {\n     double ns = 0;\n"
               << "     for (int j = 0; j < NR; ++j) ns += double(v[j].x) * double(v[j].x) + double(v[j].y) * double(v[j].y);\n"
@@ -1070,20 +1176,25 @@ std::string forward_source(const Schedule &s, const Pass &p, int precision, cons
     o << "  }\n";
     emit_ring_exit(o);
     o << "}\n";
-    return o.str();
+    std::ostringstream head;
+    emit_header(head, precision);
+    tables.declare(head);
+    return head.str() + o.str();
 }
 
 std::string backward_source(const Schedule &s, const Pass &p, int precision, int NH, const std::vector<DevOp> &ops) {
     const int RB = p.reg_bits, K = p.K, TB = K - RB;
     const int NLS = std::max(1, p.n_slots);
     const PassPlan pl = pass_plan(p.qbits, precision);
-    const int scratch = bwd_scratch(p, precision, NH), NB = bwd_buffers(p, precision, NH, scratch);
+    const BwdShape shape = bwd_shape(p, precision, NH);
+    const int scratch = shape.scratch, NB = shape.buffers;
     const int G = bwd_groups(p);
     std::vector<const StageDesc *> ex;
     for (int si = p.n_stages - 1; si >= 0; --si) ex.push_back(&s.stages[p.stage_begin + si]);
     const LayPlan lp = plan_layouts(pl, ex, TB);
-    bool pass_phase = false;
-    for (int k = 0; k < p.n_sops; ++k) pass_phase = pass_phase || leaves_factor(s.stage_ops[p.sop_begin + k]);
+    const StageOp *sops = s.stage_ops.data() + p.sop_begin;
+    const bool norm = std::any_of(sops, sops + p.n_sops, [](const StageOp &so) { return so.norm != 0; });
+    RunTables tables;
     Rows rows;
     rows.batch = scratch / (32 * elem_bytes(precision) / 2);
     rows.NH = NH;
@@ -1100,7 +1211,6 @@ std::string backward_source(const Schedule &s, const Pass &p, int precision, int
       << "  double *wacc0 = reinterpret_cast<double *>(smem + NB * BUFB + G * mtb);\n"
       << "  pipe::u64 *full = reinterpret_cast<pipe::u64 *>(wacc0 + G * WS);\n"
       << "  volatile long long *ticket = reinterpret_cast<volatile long long *>(full + NB);\n"
-      << "  V *ph = reinterpret_cast<V *>(full + 16) + int(threadIdx.x) / NT;   // factor left for the end of the pass\n"
       << "  if (threadIdx.x == 0) {\n   for (int k = 0; k < NB; ++k) {\n    pipe::mbar_init(full + k, 1);\n    ticket[k] = -1;\n   }\n"
       << "   pipe::fence_mbar_init();\n  }\n"
       << "  for (int i = int(threadIdx.x); i < G * WS; i += int(blockDim.x)) wacc0[i] = 0;\n  __syncthreads();\n"
@@ -1114,8 +1224,10 @@ std::string backward_source(const Schedule &s, const Pass &p, int precision, int
     o << "  const int warp = int(tid) / 32, lane = int(tid) % 32;\n"
       << "  V *mt = reinterpret_cast<V *>(smem + NB * BUFB + grp * mtb);\n"
       << "  double *wacc = wacc0 + grp * WS, *wrow = wacc + warp * NLS * NH;\n"
-      << "  const unsigned scr = pipe::saddr(reinterpret_cast<V *>(full + 16) + 16) + unsigned(grp * nw + warp) * "
-      << scratch << "u;\n"
+      << "  double *ph = reinterpret_cast<double *>(full + 16) + grp;\n"
+      << "  const unsigned scr = pipe::saddr(full + 32) + unsigned(grp * nw + warp) * " << scratch << "u;\n"
+      << "  V *runs = reinterpret_cast<V *>(reinterpret_cast<unsigned char *>(full + 32) + G * nw * " << scratch << ") + grp * "
+      << (shape.runs + 1) / 2 * 2 << ";\n"
       << "  long long cached_b = -1;\n"
       << "  for (long long i = grp; i < cnt; i += G) {\n"
       << "   const long long w = first + i, b = w >> a.g.n_out;\n"
@@ -1124,8 +1236,9 @@ std::string backward_source(const Schedule &s, const Pass &p, int precision, int
       << "   V *psi = reinterpret_cast<V *>(smem + sb * BUFB);\n   V *lam = psi + TS;\n"
       << "   if (b != cached_b) {\n    pipe::consumers_sync(BAR, NT);\n"
       << "    pipe::load_mtab(mt, a.mt, a.n_mt, a.mats + b * a.mats_stride, a.cpool, tid, NT);\n"
-      << "    cached_b = b;\n    pipe::consumers_sync(BAR, NT);\n"
-      << (pass_phase ? "    pipe::pass_phase(ph, mt, a.mt, a.n_mt, tid);\n    pipe::consumers_sync(BAR, NT);\n" : "") << "   }\n";
+      << "    cached_b = b;\n    pipe::consumers_sync(BAR, NT);\n";
+    emit_load_derived(o, norm, shape.runs);
+    o << "   }\n";
     emit_ring_wait(o);
     if (lp.relayout_in) {
         o << "   {\n    V *tbase = psi;\n";
@@ -1137,25 +1250,17 @@ std::string backward_source(const Schedule &s, const Pass &p, int precision, int
         const bool last = si + 1 == ex.size();
         emit_stage_load(o, pl, sd, RB, TB, NH, lp.in[si], false);
         StageCtx ctx;
-        o << "    V sc = cval<V>(1, 0);\n    R S[NH];\n";
-        for (int k = sd.op_end - 1; k >= sd.op_begin;) {
-            std::vector<const StageOp *> run;
-            std::vector<int> gids;
-            for (; k >= sd.op_begin; --k) {
-                const StageOp &so = s.stage_ops[p.sop_begin + k];
-                if (!phase_op(so, ops[so.op].gate_id, true)) break;
-                run.push_back(&so);
-                gids.push_back(ops[so.op].gate_id);
-            }
-            if (!run.empty()) {
-                emit_phase_run(o, run, gids, RB, &rows, ctx);
-            } else {
-                const StageOp &so = s.stage_ops[p.sop_begin + k--];
+        o << "    W sc = cval<W>(1, 0);\n    R S[NH];\n";
+        walk_stage(
+            sd, sops, ops, true,
+            [&](const std::vector<const StageOp *> &run, const std::vector<int> &gids) {
+                emit_phase_run(o, run, gids, RB, &rows, shape.runs ? &tables : nullptr, ctx);
+            },
+            [&](const StageOp &so) {
                 emit_backward_op(o, so, NH, ops[so.op].gate_id, rows);
                 ctx.S = ctx.S && keeps_sums(so);
-            }
-        }
-        emit_stage_phase(o, RB, true, ctx, last, last && pass_phase);
+            });
+        emit_stage_phase(o, RB, true, ctx, last, norm);
         emit_stage_store(o, pl, sd, RB, TB, NH, lp.in[si], lp.out[si], !last || lp.relayout_out);
     }
     if (int(rows.order.size()) % rows.batch) rows.flush(o);
@@ -1185,6 +1290,7 @@ std::string backward_source(const Schedule &s, const Pass &p, int precision, int
     head << "__constant__ unsigned short row_slot[" << std::max<size_t>(1, rows.order.size()) << "] = {";
     for (size_t i = 0; i < rows.order.size(); ++i) head << (i ? ", " : "") << rows.order[i];
     head << "};   // gradient row -> pass-local slot * NH + Hamiltonian\n";
+    tables.declare(head);
     return head.str() + o.str();
 }
 
@@ -1207,7 +1313,7 @@ std::string compile_input(const Entry &e, const char *const *opts, int n_opts) {
     nvrtcVersion(&major, &minor);
     std::string in = "nvrtc " + std::to_string(major) + "." + std::to_string(minor) + "\n";
     for (int i = 0; i < n_opts; ++i) in += std::string(opts[i]) + "\n";
-    for (const char *h : {kJitRegmath, kJitTile, kJitAbi, kJitPipe, kJitPhase}) in += std::string(h) + "\n";
+    for (const char *h : {kJitRegmath, kJitTile, kJitAbi, kJitPipe}) in += std::string(h) + "\n";
     return in + e.src;
 }
 
@@ -1249,9 +1355,9 @@ void compile_entry(Entry &e) {
         }
     }
     nvrtcProgram prog = nullptr;
-    const char *hdrs[5] = {kJitRegmath, kJitTile, kJitAbi, kJitPipe, kJitPhase};
-    const char *names[5] = {"regmath.cuh", "tile.cuh", "jit_abi.h", "pipe.cuh", "phasemath.cuh"};
-    if (nvrtcCreateProgram(&prog, e.src.c_str(), "mqb_pass.cu", 5, hdrs, names) != NVRTC_SUCCESS) {
+    const char *hdrs[4] = {kJitRegmath, kJitTile, kJitAbi, kJitPipe};
+    const char *names[4] = {"regmath.cuh", "tile.cuh", "jit_abi.h", "pipe.cuh"};
+    if (nvrtcCreateProgram(&prog, e.src.c_str(), "mqb_pass.cu", 4, hdrs, names) != NVRTC_SUCCESS) {
         e.log = "nvrtcCreateProgram failed";
         return;
     }
@@ -1344,6 +1450,24 @@ std::vector<const void *> kernels_for(const std::vector<std::string> &srcs) {
 
 }  // namespace
 
+int jit_run_entries(const std::vector<const StageDesc *> &stages, const StageOp *sops, const std::vector<DevOp> &ops,
+                    int precision, bool adj) {
+    if (precision != MQB_PREC_C64) return 0;
+    RunTables tables;
+    for (const StageDesc *sd : stages)
+        walk_stage(
+            *sd, sops, ops, adj,
+            [&](const std::vector<const StageOp *> &run, const std::vector<int> &gids) {
+                std::vector<const StageOp *> same;
+                std::vector<int> bits;
+                for (size_t k = 0; k < run.size(); ++k)
+                    if (RunTables::takes(*run[k], gids[k])) same.push_back(run[k]);
+                tables.add(same, bits);
+            },
+            [](const StageOp &) {});
+    return int(tables.entries.size());
+}
+
 std::string jit_forward_source(const Schedule &s, const Pass &p, int precision, const std::vector<DevOp> &ops) {
     return forward_source(s, p, precision, ops);
 }
@@ -1395,8 +1519,8 @@ size_t jit_forward_smem(const Pass &p, int precision) { return fwd_smem(p, preci
 
 size_t jit_backward_smem(const Pass &p, int precision, int n_hams) {
     const size_t buf = (size_t(1) << p.K) * elem_bytes(precision) * (1 + n_hams);
-    const int scratch = bwd_scratch(p, precision, n_hams);
-    return size_t(bwd_buffers(p, precision, n_hams, scratch)) * buf + bwd_fixed_smem(p, precision, n_hams, scratch);
+    const BwdShape b = bwd_shape(p, precision, n_hams);
+    return size_t(b.buffers) * buf + bwd_fixed_smem(p, precision, n_hams, b.scratch, b.runs);
 }
 
 namespace {

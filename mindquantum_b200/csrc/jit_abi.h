@@ -39,9 +39,7 @@ struct JitMtab {
     int mcount;             // entries (M, then dM_0, dM_1, ...)
     long long msrc;         // offset in the per-sample block or the constant pool
     int msrc_ps;            // 1: per-sample matrices, 0: constant pool
-    int phase;              // bits 0-1: a unit-modulus diagonal pair (kPhaseUniform 1, kPhasePair 2) whose second entry
-                            // becomes the ratio to the first (phasemath.cuh); bits 8..: entries that measure
-                            // the gate's norm (0: not measured), bit 7: of a diagonal
+    int norm;               // rows of M (2 or 4; negative: a diagonal) where the gate's norm is measured, else 0
 };
 
 template <typename V>

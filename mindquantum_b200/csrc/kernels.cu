@@ -320,14 +320,6 @@ __global__ void matgen_kernel(MatgenArgs a) {
         }
         GateMats gm;
         gate_mats(op.gate_id, t, gm);
-        if (sizeof(R) == 4 && a.ratios && (op.gate_id == GID_RZ || op.gate_id == GID_RZZ)) {
-            // what the state sees is the ratio of the two phases, e^{i t}: take the second from the rounded first, so
-            // that complex64 rounds the ratio once instead of twice the half angle
-            const double ar = double(float(gm.M[0].x)), ai = double(float(gm.M[0].y));
-            const double w = 1.0 / sqrt(ar * ar + ai * ai), c = cos(t[0]), s = sin(t[0]);
-            gm.M[1] = z2((ar * c - ai * s) * w, (ar * s + ai * c) * w);
-            if (op.gate_id == GID_RZZ) gm.M[2] = gm.M[1];
-        }
         for (int e = 0; e < op.mat_size; ++e) out[op.mat_off + e] = cvt<V>(gm.M[e]);
         if (op.grad_mask)
             for (int an = 0; an < op.n_angles; ++an)

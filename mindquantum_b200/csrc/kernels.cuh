@@ -31,7 +31,6 @@ struct MatgenArgs {
     int64_t batch;
     void *mats;                // per-sample matrices (cplx<R>)
     int64_t mats_stride;       // complex entries per sample
-    int ratios;                // the matrices are for generated passes, which read a diagonal pair by its ratio
 };
 
 template <typename R>

@@ -121,15 +121,9 @@ struct StageOp {
     int32_t code;        // RegCode of the forward kernels
     int32_t bcode;       // code * 4 + gradient selector, for the backward kernels
     int32_t cflags;      // bit 0: octrl != 0, bit 1: tctrl != 0 (controls checked per thread)
-    int32_t phase;       // generated kernels: a StagePhase kind, and kPhaseUnitary
+    int16_t unitary;     // DevOp::unitary != 0
+    int16_t norm;        // JitMtab::norm
 };
-
-// StageOp::phase, for the generated kernels: a diagonal gate whose table holds the ratio of its pair, with the
-// first entry the same for every thread, so that it waits for the end of the pass (kPhaseUniform: uncontrolled,
-// on register bits, or a global phase), or not (kPhasePair); a flag of the gates known to be unitary; and from bit
-// kPhaseNormShift on, for the uncontrolled gates of a complex64 pass, the entries of M whose mean square says by
-// how much rounding took the gate away from norm one (0: not counted; kPhaseDiag: they are a diagonal's).
-enum StagePhase : int32_t { kPhaseUniform = 1, kPhasePair = 2, kPhaseKind = 3, kPhaseUnitary = 4, kPhaseDiag = 128, kPhaseNormShift = 8 };
 
 // A pass: one sweep over the state(s).
 struct Pass {
@@ -146,6 +140,7 @@ struct Pass {
     int mtab_entries = 0;                    // fused: complex entries of the pass's shared-memory matrix table
     // the forward kernel's own stage layout of the same pass (more register bits, no lambdas)
     int f_stage_begin = 0, f_n_stages = 0, f_sop_begin = 0, f_n_sops = 0, f_mtab_entries = 0, f_reg_bits = 0;
+    int run_entries = 0, f_run_entries = 0;  // generated kernels: entries of the shared tables of runs (jit_run_entries)
     int reg_bits = 0, thread_bits = 0;       // fused: registers / threads of the tile kernel
 };
 
@@ -202,6 +197,11 @@ class JitBlock {
   private:
     bool prev_;
 };
+
+// Entries of the factor tables that a generated kernel of a pass keeps in shared memory for its runs of diagonal
+// gates: `stages` in execution order, `sops` the pass's stage ops (jit.cpp).
+int jit_run_entries(const std::vector<const StageDesc *> &stages, const StageOp *sops, const std::vector<DevOp> &ops,
+                    int precision, bool adj);
 
 // What one fused pass may hold besides kMaxPassOps and kMaxPassSlots.
 struct PassLimits {

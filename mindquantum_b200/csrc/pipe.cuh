@@ -9,7 +9,7 @@
 #define MQB_PIPE_CUH_
 
 #include "jit_abi.h"
-#include "phasemath.cuh"
+#include "regmath.cuh"
 
 namespace mqb {
 namespace pipe {
@@ -104,8 +104,7 @@ __device__ __forceinline__ bool consumers_and(int id, int n, bool q) {
     return r != 0;
 }
 
-// The matrices of a pass's ops into shared memory, by the nt consumer threads (one warp per op), with the
-// ratios of the diagonal pairs.
+// The matrices of a pass's ops into shared memory, by the nt consumer threads (one warp per op).
 template <typename V>
 __device__ __forceinline__ void load_mtab(V *mtab, const JitMtab *mt, int n, const V *mb, const V *cpool, unsigned tid,
                                           unsigned nt) {
@@ -114,51 +113,78 @@ __device__ __forceinline__ void load_mtab(V *mtab, const JitMtab *mt, int n, con
         const JitMtab e = mt[k];
         const V *src = (e.msrc_ps ? mb : cpool) + e.msrc;
         for (int i = static_cast<int>(lane); i < e.mcount; i += 32) mtab[e.moff + i] = src[i];
-        if (e.phase & 3) {
-            __syncwarp();
-            if (lane == 0) reg::prepare_pair(mtab + e.moff);
-        }
     }
 }
 
-// The factor left for the end of a pass, made by the group's first warp after the table is complete: the product
-// of the uniform diagonal pairs' first entries, over the norms that rounding gave the uncontrolled gates.  A
-// complex64 rotation's c and s leave c^2 + s^2 off one by some 1e-8, the same for every amplitude, so over
-// hundreds of gates the state's norm drifted by 1e-6 and took the expectation and the gradients along; one
-// factor per pass takes it out.
+__device__ __forceinline__ double2 wide(float2 a) { return make_double2(a.x, a.y); }
+__device__ __forceinline__ double2 wide(double2 a) { return a; }
+
+// The factor of a value of a run's register bits: in a forward pass as the sum of two complex64 numbers, so that the run
+// loses nothing by its table; in the adjoint, whose result is less sensitive, rounded once.
+struct alignas(16) Split {
+    float2 hi, lo;
+};
+__device__ __forceinline__ float2 times(float2 a, const Split &t) {
+    float2 r;
+    r.x = fma(-a.y, t.hi.y, fma(a.x, t.hi.x, fma(-a.y, t.lo.y, a.x * t.lo.x)));
+    r.y = fma(a.y, t.hi.x, fma(a.x, t.hi.y, fma(a.y, t.lo.x, a.x * t.lo.y)));
+    return r;
+}
+__device__ __forceinline__ float2 times(float2 a, float2 t) { return reg::cmul(a, t); }
+__device__ __forceinline__ void put_factor(Split &t, double2 p) {
+    t.hi = make_float2(float(p.x), float(p.y));
+    t.lo = make_float2(float(p.x - double(t.hi.x)), float(p.y - double(t.hi.y)));
+}
+__device__ __forceinline__ void put_factor(float2 &t, double2 p) { t = make_float2(float(p.x), float(-p.y)); }   // of U^dag
+
+// A gate of a run: M at moff, its targets' places among the run's bits (-1: no such target), its controls.
+struct RunGate {
+    unsigned short moff;
+    signed char p0, p1;
+    unsigned char ctrl;
+};
+// An entry of a run's table: the product of n gates' entries for the bits idx.
+struct RunEntry {
+    unsigned short first;
+    unsigned char n, idx;
+};
+
+// The tables of a pass's runs from its matrix table, by the nt threads of a group, the products in FP64.
+template <typename T, typename V>
+__device__ __forceinline__ void load_runs(T *runs, const V *mtab, const RunGate *gates, const RunEntry *entries, int n,
+                                          unsigned tid, unsigned nt) {
+    for (unsigned e = tid; e < unsigned(n); e += nt) {
+        const RunEntry en = entries[e];
+        double2 p = make_double2(1, 0);
+        for (int k = 0; k < en.n; ++k) {
+            const RunGate g = gates[en.first + k];
+            if ((en.idx & g.ctrl) != g.ctrl) continue;
+            const int r = (g.p0 < 0 ? 0 : en.idx >> g.p0 & 1) | (g.p1 < 0 ? 0 : (en.idx >> g.p1 & 1) << 1);
+            p = reg::cmul(p, wide(mtab[g.moff + r]));
+        }
+        put_factor(runs[e], p);
+    }
+}
+
+// One over the norm that rounding gave the uncontrolled gates of a pass, by the group's first warp after the matrix table
+// is complete.  A complex64 rotation's c and s leave c^2 + s^2 off one by some 1e-8, the same for every
+// amplitude, so over hundreds of gates the state's norm drifts by 1e-6 and takes the expectation and the
+// gradients along; one factor per pass takes it out.
 template <typename V>
-__device__ __forceinline__ void pass_phase(V *ph, const V *mtab, const JitMtab *mt, int n, unsigned tid) {
+__device__ __forceinline__ void pass_norm(double *ph, const V *mtab, const JitMtab *mt, int n, unsigned tid) {
     if (tid >= 32u) return;
-    double2 p = reg::cval<double2>(1, 0);
+    double p = 1;
     for (int k = static_cast<int>(tid); k < n; k += 32) {
         const JitMtab e = mt[k];
+        if (e.norm == 0) continue;
+        const int rows = e.norm < 0 ? -e.norm : e.norm, cnt = e.norm < 0 ? rows : rows * rows;
         const V *M = mtab + e.moff;
-        const int kind = e.phase & 3, norm = e.phase >> 8;
-        double q = 1;   // mean square of what the gate multiplies amplitudes by
-        auto sq = [&](int i) { return double(M[i].x) * double(M[i].x) + double(M[i].y) * double(M[i].y); };
-        if (kind == 1) p = reg::cmul(p, reg::unit(reg::wide(M[0])));
-        if (norm) {
-            if (kind == 1) {            // (1, r)
-                q = 0.5 * (1.0 + sq(1));
-            } else if (kind == 2) {     // d0 = M[0] or M[2], times (1, r) or (1, conj r)
-                q = 0.25 * (sq(0) + sq(2)) * (1.0 + sq(1));
-            } else {                    // 4^m entries of 2^m rows, or a diagonal of 2^m
-                q = 0;
-                for (int i = 0; i < norm; ++i) q += sq(i);
-                q /= e.phase & 128 ? norm : norm == 16 ? 4 : 2;
-            }
-            const double t = 1.5 - 0.5 * q;   // 1 / sqrt(q) for q this close to one
-            p.x *= t;
-            p.y *= t;
-        }
+        double q = 0;   // mean square of what the gate multiplies amplitudes by
+        for (int i = 0; i < cnt; ++i) q += double(M[i].x) * double(M[i].x) + double(M[i].y) * double(M[i].y);
+        p *= 1.5 - 0.5 * (q / rows);   // 1 / sqrt(q) for q this close to one
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        double2 q;
-        q.x = __shfl_xor_sync(0xffffffffu, p.x, o);
-        q.y = __shfl_xor_sync(0xffffffffu, p.y, o);
-        p = reg::cmul(p, q);
-    }
-    if (tid == 0u) *ph = reg::cval<V>(p.x, p.y);
+    for (int o = 16; o > 0; o >>= 1) p *= __shfl_xor_sync(0xffffffffu, p, o);
+    if (tid == 0u) *ph = p;
 }
 
 // Gradient rows of a warp: shared scratch at `scr` holds N = 4 or 8 rows of 32 float partials, or 2 of double.

@@ -538,24 +538,20 @@ void build_stages(Schedule &s, const std::vector<DevOp> &ops, int reg_bits, int 
                     }
                 }
                 assign_codes(so);
-                if (dop.unitary) {
-                    so.phase = kPhaseUnitary;
-                    const bool reg0 = so.dsrc[0] == 0, reg1 = so.dsrc[1] == 0;
-                    const bool one = so.kind == SK_DIAG1 && reg0, zz = so.kind == SK_DIAG2 && dop.gate_id == GID_RZZ;
-                    if ((so.kind == SK_DIAG1 && dop.gate_id == GID_GP) || one || (zz && reg0 && reg1))
-                        so.phase |= dop.ctrl ? (one && !so.rctrl && dop.gate_id != GID_GP ? kPhasePair : 0) : kPhaseUniform;
-                    else if (zz && (reg0 || reg1) && !so.rctrl)
-                        so.phase |= kPhasePair;
-                    if (zz && reg0 && reg1 && dop.ctrl && !so.rctrl) so.phase |= kPhasePair;
-                    // (of the constant matrices only the first gate on a qubit counts: on the structured states of
-                    // Clifford circuits the roundings of later ones cancel)
-                    if (precision == MQB_PREC_C64 && !dop.ctrl && so.kind != SK_SWAP1 && (dop.per_sample || dop.unitary == 2)) so.phase |= dop.mat_size << kPhaseNormShift | (so.kind == SK_DIAG1 || so.kind == SK_DIAG2 ? kPhaseDiag : 0);
-                }
+                so.unitary = dop.unitary != 0;
+                // the norm that rounding gave an uncontrolled complex64 gate is measured (of the constant matrices only the
+                // first gate's on a qubit: on the structured states of Clifford circuits the later ones cancel)
+                if (precision == MQB_PREC_C64 && !dop.ctrl && so.kind != SK_SWAP1 && (dop.unitary == 2 || (dop.unitary && dop.per_sample)))
+                    so.norm = int16_t(so.kind == SK_DIAG1 ? -2 : so.kind == SK_DIAG2 ? -4 : so.kind == SK_DENSE2 ? 4 : 2);
                 stage_ops.push_back(so);
             }
             sd.op_end = int(stage_ops.size()) - sop_begin;
             stages.push_back(sd);
         }
+        std::vector<const StageDesc *> order;   // of execution
+        for (size_t k = size_t(stage_begin); k < stages.size(); ++k) order.push_back(&stages[k]);
+        if (!forward) std::reverse(order.begin(), order.end());
+        (forward ? p.f_run_entries : p.run_entries) = jit_run_entries(order, stage_ops.data() + sop_begin, ops, precision, !forward);
         if (forward) {
             p.f_reg_bits = RB;
             p.f_stage_begin = stage_begin;
