@@ -195,6 +195,7 @@ struct SchedDev {
     std::map<int, std::vector<const void *>> jit_bwd; // generated backward kernels, by lambdas
     SmallOp *d_small = nullptr;                       // the gates in execution order, when the block-per-sample kernel runs them
     size_t small_smem = 0;                            // its shared memory (0: the tile kernels run)
+    int small_saved = 0;                              // states per sample that it keeps for its backward sweep
     ~SchedDev() {
         cudaFree(d_small);
         cudaFree(d_jmt);
@@ -301,8 +302,7 @@ constexpr int kSmallMaxQubits = 10;
 constexpr int kSmallAnyBatchQubits = 8;
 
 // The block-per-sample kernel's gate list, in the schedule's execution order, when it can run the
-// program: gates of at most two targets, unitary where a gradient undoes them, everything in one
-// block's shared memory.  Callers that force a kernel family (jit, tile_bits, fuse) get that one.
+// program: gates of at most two targets, everything in one block's shared memory.  Callers that force a kernel family (jit, tile_bits, fuse) get that one.
 static void plan_small(const mqb_program &p, SchedDev &sd, int n_hams) {
     if (!p.fuse || p.jit != 0 || p.tile_bits != 0 || p.n > kSmallMaxQubits || p.ops.empty()) return;
     if (n_hams > 0 && p.nonunitary) return;
@@ -328,6 +328,7 @@ static void plan_small(const mqb_program &p, SchedDev &sd, int n_hams) {
             so.mat_size = op.mat_size;
             so.grad_mask = op.grad_mask;
             so.slot0 = op.slot0;
+            if (n_hams > 0 && !op.unitary) so.save = int16_t(++sd.small_saved);
             const int done = q + 1;
             // norm checks as grad_layout places them: after pass `done`, and of the state before pass q
             if (i + 1 == ps.op_end && (done % sn == 0 || done == P)) so.check |= 1;
@@ -344,8 +345,12 @@ static std::unique_ptr<SchedDev> make_sched(const mqb_program &p, int K, bool fu
     // the register kernels need 2^5..2^8 threads of 2^reg_bits amplitudes: smaller registers use
     // the per-gate kernels
     if (K < reg_bits + 5) fuse = false;
-    sd->s = build_schedule(p.n, K, contiguity_bits(p.precision), p.ops, fuse, &p.apart,
-                           pass_limits(p, K, reg_bits, n_hams));
+    std::vector<char> apart = p.apart;
+    // a gradient undoes a pass by its gates' conjugate transposes: a constant matrix that is not unitary takes the stored
+    // state before its pass, and no gate with a gradient shares that pass
+    for (size_t k = 0; n_hams > 0 && k < apart.size(); ++k)
+        if (p.descs[k].gate_id == GID_MATRIX && !p.ops[k].unitary) apart[k] = 1;
+    sd->s = build_schedule(p.n, K, contiguity_bits(p.precision), p.ops, fuse, &apart, pass_limits(p, K, reg_bits, n_hams));
     build_stages(sd->s, p.ops, reg_bits, p.precision, false);
     build_stages(sd->s, p.ops, p.use_jit() ? jit_fwd_reg_bits(p.precision) : fwd_reg_bits(p.precision), p.precision, true);
     sd->s.d_pass_ops = upload(sd->s.pass_ops);
@@ -463,11 +468,12 @@ static void run_matgen(const mqb_program &p, const double *params, int64_t param
 }
 
 // Whether a call runs the block-per-sample kernel: the schedule has it, and the tile kernels either cannot
-// fuse this register or are not the faster ones at this batch.
+// fuse this register or are not the faster ones at this batch, or undo gates that they should not (a custom gate, whose
+// matrices the caller makes: its evaluation on the host takes longer than either kernel).
 static bool runs_small(const mqb_program &p, const SchedDev &sd, int64_t batch) {
     if (!sd.small_smem) return false;
     const bool tiles = std::any_of(sd.s.passes.begin(), sd.s.passes.end(), [](const Pass &ps) { return ps.fused != 0; });
-    return !tiles || p.n <= kSmallAnyBatchQubits || batch <= 2 * int64_t(sm_count_cached());
+    return !tiles || sd.small_saved || p.n <= kSmallAnyBatchQubits || batch <= 2 * int64_t(sm_count_cached());
 }
 
 template <typename R, typename S>
@@ -606,7 +612,7 @@ static void ham_impl(const mqb_hamiltonian &h, const cplx<R> *bra, const cplx<R>
 }
 
 struct GradLayout {
-    size_t mats = 0, gslots = 0, lam = 0, w = 0, ckpt = 0, norms = 0, total = 0;
+    size_t mats = 0, gslots = 0, lam = 0, w = 0, ckpt = 0, norms = 0, saved = 0, total = 0;
     int n_ckpt = 0;
     bool need_w = false;
     std::vector<int> ckpt_index;   // p (1..P) -> checkpoint buffer index or -1
@@ -615,8 +621,10 @@ struct GradLayout {
     std::vector<int> norm_fwd, norm_bwd;
 };
 
-static GradLayout grad_layout(const mqb_program &p, const Schedule &s, int64_t batch, int n_hams, int stride, bool small) {
+static GradLayout grad_layout(const mqb_program &p, const SchedDev &sd, int64_t batch, int n_hams, int stride) {
     GradLayout L;
+    const Schedule &s = sd.s;
+    const bool small = sd.small_smem != 0;
     const int P = int(s.passes.size());
     const size_t state = (size_t(1) << p.n) * p.elem() * batch;
     L.ckpt_index.assign(P + 1, -1);
@@ -642,7 +650,8 @@ static GradLayout grad_layout(const mqb_program &p, const Schedule &s, int64_t b
     L.w = L.need_w ? align_up(state) : 0;
     L.ckpt = align_up(state) * L.n_ckpt;
     L.norms = align_up((L.norm_fwd.size() + L.norm_bwd.size()) * size_t(batch) * 2 * sizeof(double));
-    L.total = L.mats + L.gslots + L.lam + L.w + L.ckpt + L.norms;
+    L.saved = align_up((size_t(sd.small_saved) << p.n) * size_t(batch) * sizeof(double2));
+    L.total = L.mats + L.gslots + L.lam + L.w + L.ckpt + L.norms + L.saved;
     return L;
 }
 
@@ -660,7 +669,7 @@ static void grad_impl(mqb_program &p, const mqb_hamiltonian *const *hams, int n_
              stride);
     SchedDev &sd = grad_schedule(p, n_hams);
     const Schedule &s = sd.s;
-    const GradLayout L = grad_layout(p, s, batch, n_hams, stride, sd.small_smem != 0);
+    const GradLayout L = grad_layout(p, sd, batch, n_hams, stride);
     if (ws == nullptr || ws_bytes < L.total) fail(MQB_ERR_WORKSPACE, "workspace too small (%zu < %zu)", ws_bytes, L.total);
     unsigned char *base = static_cast<unsigned char *>(ws);
     V *mats = reinterpret_cast<V *>(base);
@@ -697,6 +706,7 @@ static void grad_impl(mqb_program &p, const mqb_hamiltonian *const *hams, int n_
         a.scale = lam_in ? 1.0 : 2.0;
         // the sweep rebuilds every state; the checks it keeps are those of this stride's layout
         a.norms = L.norms ? reinterpret_cast<double *>(ck0 + L.ckpt) : nullptr;
+        a.saved = L.saved ? reinterpret_cast<cplx<double> *>(ck0 + L.ckpt + L.norms) : nullptr;
         a.ckpt_stride = stride;
         TimeScope ts(TK_BWD, st);
         ck((launch_small<double, R>(a, sd.small_smem, st)), "small register gradient");
@@ -1496,7 +1506,7 @@ int mqb_grad_workspace_size(const mqb_program *p, int64_t batch, int n_hams, int
         if (n_hams < 1) fail(MQB_ERR_INVALID, "need at least one Hamiltonian");
         if (batch < 1) fail(MQB_ERR_INVALID, "batch must be >= 1");
         SchedDev &sd = grad_schedule(const_cast<mqb_program &>(*p), n_hams);
-        *bytes = grad_layout(*p, sd.s, batch, n_hams, stride, sd.small_smem != 0).total;
+        *bytes = grad_layout(*p, sd, batch, n_hams, stride).total;
     });
 }
 
@@ -1507,7 +1517,7 @@ int mqb_grad_norm_checks(mqb_program *p, const void *ws, size_t ws_bytes, int64_
         if (!p || !n_checks) fail(MQB_ERR_INVALID, "null argument");
         if (n_hams < 1 || batch < 1) fail(MQB_ERR_INVALID, "invalid batch or number of Hamiltonians");
         SchedDev &sd = grad_schedule(*p, n_hams);
-        const GradLayout L = grad_layout(*p, sd.s, batch, n_hams, stride, sd.small_smem != 0);
+        const GradLayout L = grad_layout(*p, sd, batch, n_hams, stride);
         const int n = int(L.norm_fwd.size() + L.norm_bwd.size());
         *n_checks = n;
         if (n == 0 || !out) return;

@@ -3,7 +3,8 @@
 // A block owns one sample.  It copies the gate records and the sample's matrices into shared memory,
 // runs the gates on the state there (a thread per amplitude pair, one barrier per gate), and for a
 // gradient applies the Hamiltonians and runs the adjoint sweep on psi and every lambda in the same
-// launch, down to the parameters.  Nothing but the results is written.
+// launch, down to the parameters.  Nothing but the results is written (and the states before gates that are not known to be
+// unitary, which the sweep reads back).
 //
 // Why a kernel of its own: the tile kernels hold 2^RB amplitudes in each thread of at least one warp, so
 // the smallest registers ran one kernel per gate (a 6-qubit classifier's training step on 32 samples: 310
@@ -147,6 +148,11 @@ __global__ void __launch_bounds__(kSmallThreads) small_kernel(const SmallArgs<R,
     for (int k = 0; k < a.n_ops; ++k) {
         const SmallOp &op = sops[k];
         const V *M = mt + op.moff;
+        if (op.save) {
+            V *keep = a.saved + ((op.save - 1) * a.batch + b) * dim;
+            for (unsigned i = tid; i < dim; i += T) keep[i] = psi[i];
+            __syncthreads();
+        }
         if (op.m == 1) {
             const unsigned bit = 1u << op.t0;
             for (unsigned g = tid; g < dim / 2; g += T) {
@@ -214,12 +220,17 @@ __global__ void __launch_bounds__(kSmallThreads) small_kernel(const SmallArgs<R,
         }
     }
     __syncthreads();
-    // adjoint sweep: psi <- U^dag psi, slot += Re <lambda| dU |psi>, lambda <- U^dag lambda
+    // adjoint sweep: psi <- U^dag psi (or the kept state), slot += Re <lambda| dU |psi>, lambda <- U^dag lambda
     int par = 0;
     for (int k = a.n_ops - 1; k >= 0; --k) {
         const SmallOp &op = sops[k];
         const V *M = mt + op.moff;
         const int G = op.grad_mask;
+        if (op.save) {
+            const V *keep = a.saved + ((op.save - 1) * a.batch + b) * dim;
+            for (unsigned i = tid; i < dim; i += T) psi[i] = keep[i];
+            __syncthreads();
+        }
         double acc[3][kSmallMaxHams];
 #pragma unroll
         for (int an = 0; an < 3; ++an)
@@ -231,7 +242,7 @@ __global__ void __launch_bounds__(kSmallThreads) small_kernel(const SmallArgs<R,
                 const unsigned i = group_base(op, g);
                 if ((i & op.ctrl) != op.ctrl) continue;
                 V x0 = psi[i], x1 = psi[i | bit];
-                gate1<V, true>(op, M, x0, x1);
+                if (!op.save) gate1<V, true>(op, M, x0, x1);
                 psi[i] = x0;
                 psi[i | bit] = x1;
 #pragma unroll
@@ -264,7 +275,7 @@ __global__ void __launch_bounds__(kSmallThreads) small_kernel(const SmallArgs<R,
                 if ((i & op.ctrl) != op.ctrl) continue;
                 const unsigned id[4] = {i, i | (1u << op.t0), i | (1u << op.t1), i | (1u << op.t0) | (1u << op.t1)};
                 V x[4] = {psi[id[0]], psi[id[1]], psi[id[2]], psi[id[3]]};
-                gate2<V, true>(op, M, x);
+                if (!op.save) gate2<V, true>(op, M, x);
 #pragma unroll
                 for (int r = 0; r < 4; ++r) psi[id[r]] = x[r];
 #pragma unroll

@@ -10,7 +10,9 @@ constexpr int kSmallMaxHams = 4;
 
 // One gate of the small-register kernel, in execution order.
 struct SmallOp {
-    int32_t kind, m, sub;        // OpKind, targets, DenseSub
+    int16_t kind, m, sub;        // OpKind, targets, DenseSub
+    int16_t save;                // gradient: 1 + the place of the state before the gate, kept because its conjugate transpose
+                                 // does not undo it (0: it does)
     int32_t t0, t1;              // target qubits (matrix bits 0 and 1)
     uint32_t ctrl;               // control mask
     int32_t moff;                // M in the block's matrix table: the per-sample block, then the constant pool
@@ -52,6 +54,7 @@ struct SmallArgs {
     const double *csr_coeff;
     double scale;
     double *norms;               // [check][batch][2], or nullptr (no checks)
+    cplx<R> *saved;              // [SmallOp::save - 1][batch][2^n]
     int ckpt_stride;             // the states the caller's layout counts as stored have no backward check
 };
 
