@@ -611,6 +611,13 @@ class MQVectorB200(BackendBase):
         Returns:
             f: float64 [batch][n_hams][2] (re, im); grad: float64 [batch][n_hams][n_params].
         """
+        f, g, _ = self._expectation_with_grad(hams, circuit, params, param_names, grad_names, init_state, ckpt_stride)
+        return f, g[:, :, :len(param_names)]
+
+    def _expectation_with_grad(self, hams, circuit, params, param_names, grad_names=None, init_state=None,
+                               ckpt_stride=None, joint=False):
+        """f, grad (n_params or 1 columns) and, when ``joint``, the one buffer that holds f and then grad, for a
+        caller who copies both to the host at once."""
         prog = lowered(circuit, self.n_qubits, self.precision, param_names, grad_names, self.fuse, jit=self.jit)
         nh = [native_ham(h, self.n_qubits, self.precision) for h in hams]
         params = params.to(device=self.device, dtype=torch.float64).contiguous()
@@ -630,17 +637,20 @@ class MQVectorB200(BackendBase):
         released = last[2] if last is not None and last[5] == 1 else 0
         last = None
         stride, ws = self._grad_workspace(prog, batch, len(nh), ckpt_stride, released=released)
-        # f and g share one buffer, so that a caller who wants both on the host copies once
-        n_f, n_p = batch * len(nh) * 2, max(1, len(param_names))
-        fg = torch.empty(n_f + batch * len(nh) * n_p, dtype=torch.float64, device=self.device)
-        f = fg[:n_f].view(batch, len(nh), 2)
-        g = fg[n_f:].view(batch, len(nh), n_p)
+        shape_f, shape_g, fg = (batch, len(nh), 2), (batch, len(nh), max(1, len(param_names))), None
+        if joint:
+            n_f = math.prod(shape_f)
+            fg = torch.empty(n_f + math.prod(shape_g), dtype=torch.float64, device=self.device)
+            f, g = fg[:n_f].view(shape_f), fg[n_f:].view(shape_g)
+        else:
+            f = torch.empty(shape_f, dtype=torch.float64, device=self.device)
+            g = torch.empty(shape_g, dtype=torch.float64, device=self.device)
         N.call('mqb_expectation_with_grad', prog.handle, ham_arr, len(nh), _ptr(init), init_batched, batch,
                _ptr(params), params.shape[1] if params.dim() == 2 else 0, _ptr(custom), _ptr(f), _ptr(g), stride,
                _ptr(ws), ws.numel(), _stream())
         # the workspace keeps this call's FP64 norm checks until the next call (norm_checks())
         self._last_grad = (prog, ws, ws.numel(), batch, len(nh), stride)
-        return f, g[:, :, :len(param_names)]
+        return f, g, fg
 
     def norm_checks(self):
         """<psi|psi> in FP64 at the norm checks of the last complex64 gradient call: [checks][batch].
@@ -749,9 +759,9 @@ class MQVectorB200(BackendBase):
             enc, ans = _split_inputs(version, enc_names, ans_names, inputs_)
             params = np.concatenate([enc, np.broadcast_to(ans, (enc.shape[0], ans.size))], axis=1)
             init = sim._state
-            f, g = sim.expectation_with_grad_tensor(hams, circ_right, torch.as_tensor(params), names, init_state=init)
-            host = f._base.cpu().numpy()   # pylint: disable=protected-access
-            f, g = host[:f.numel()].reshape(f.shape), host[f.numel():].reshape(f.shape[0], f.shape[1], -1)[:, :, :len(names)]
+            f, g, fg = sim._expectation_with_grad(hams, circ_right, torch.as_tensor(params), names, init_state=init, joint=True)   # pylint: disable=protected-access
+            host = fg.cpu().numpy()
+            f, g = host[:f.numel()].reshape(f.shape), host[f.numel():].reshape(g.shape)[:, :, :len(names)]
             if sim.precision == N.MQB_PREC_C64 and sim._last_grad[5] != 1:
                 # states rebuilt by reverse application: report a norm that moved
                 drift = sim.norm_drift() if init is None else 0.0
