@@ -272,7 +272,7 @@ cudaError_t launch_fused_fwd2(const Fwd2Args<R> &a, int sm_count, cudaStream_t s
 #define MQB_F2(RBV)                                                                                         \
     case RBV: {                                                                                             \
         auto kern = fused_fwd2_kernel<R, RBV>;                                                              \
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)); \
+        cudaError_t e = allow_smem<fused_fwd2_kernel<R, RBV>>();                                            \
         if (e != cudaSuccess) return e;                                                                     \
         kern<<<blocks_for2(kern, threads, smem, sm_count, work), threads, smem, s>>>(a);                    \
         return cudaGetLastError();                                                                          \
@@ -304,7 +304,7 @@ cudaError_t launch_fused_bwd2(const Bwd2Args<R> &a, int sm_count, cudaStream_t s
 #define MQB_B2K(RBV, NHV)                                                                                   \
     case RBV * 8 + NHV: {                                                                                   \
         auto kern = fused_bwd2_kernel<R, RBV, NHV>;                                                         \
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)); \
+        cudaError_t e = allow_smem<fused_bwd2_kernel<R, RBV, NHV>>();                                       \
         if (e != cudaSuccess) return e;                                                                     \
         kern<<<blocks_for2(kern, threads, smem, sm_count, work), threads, smem, s>>>(a);                    \
         return cudaGetLastError();                                                                          \

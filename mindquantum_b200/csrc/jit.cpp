@@ -1578,7 +1578,8 @@ int *g_err_word[64] = {nullptr};
 
 cudaError_t launch_pipe(const void *kernel, void **argv, int threads, size_t smem, int sm_count, long long work,
                         cudaStream_t st) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    // the same for every launch: passes that share a kernel may differ in size
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 << 10);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1)

@@ -834,7 +834,7 @@ cudaError_t launch_ham_ring(const HamArgs<R> &a, const HamRingGeom &rg, const vo
     const size_t smem = ham_ring_smem(a.g, int(sizeof(cplx<R>)), threads, a.n_classes, a.n_terms,
                                       a.accumulate && a.out && rg.stage_prev, rg.nb);
     auto kern = ham_ring_kernel<R, kHamRegBits>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = allow_smem<ham_ring_kernel<R, kHamRegBits>>();
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) != cudaSuccess || per_sm < 1)
@@ -869,7 +869,7 @@ cudaError_t launch_ham(const HamArgs<R> &a, int sm_count, cudaStream_t s) {
                                        a.accumulate && a.out);
         if (smem2 <= 160 * 1024) {
             auto kern = ham2_kernel<R, kHamRegBits>;
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem2));
+            cudaError_t e = allow_smem<ham2_kernel<R, kHamRegBits>>();
             if (e != cudaSuccess) return e;
             int per_sm = 0;
             if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem2) != cudaSuccess || per_sm < 1)
@@ -882,7 +882,7 @@ cudaError_t launch_ham(const HamArgs<R> &a, int sm_count, cudaStream_t s) {
     }
     const size_t smem = ham_smem(a.g, sizeof(cplx<R>));
     auto kern = ham_kernel<R>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = allow_smem<ham_kernel<R>>();
     if (e != cudaSuccess) return e;
     const int64_t work = a.batch << a.g.n_out;
     kern<<<blocks_for(kern, smem, sm_count, work), kThreads, smem, s>>>(a);

@@ -2,6 +2,8 @@
 #ifndef MQB_KERNELS_CUH_
 #define MQB_KERNELS_CUH_
 
+#include <atomic>
+
 #include "mqb_internal.h"
 
 namespace mqb {
@@ -18,6 +20,23 @@ struct CT<double> {
 };
 template <typename R>
 using cplx = typename CT<R>::T;
+
+// Lets launches of Kern ask for all of a block's shared memory.  The limit belongs to the function, for every thread of the
+// process, while the size of a launch follows its circuit: set to each launch's own size, another thread's smaller
+// circuit could lower it between a launch's setting and the launch, which then failed.  Once per device, the same for all.
+constexpr int kMaxBlockSmem = 227 << 10;
+template <auto Kern>
+cudaError_t allow_smem() {
+    static std::atomic<uint64_t> done{0};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const uint64_t bit = dev < 64 ? uint64_t(1) << dev : 0;
+    if (done.load() & bit) return cudaSuccess;
+    e = cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
+    if (e == cudaSuccess) done.fetch_or(bit);
+    return e;
+}
 
 struct MatgenArgs {
     const DevOp *ops;

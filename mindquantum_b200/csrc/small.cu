@@ -361,7 +361,7 @@ size_t small_smem(int n, int elem_bytes, int n_hams, int n_ops, int64_t table_en
 
 template <typename R, typename S>
 cudaError_t launch_small(const SmallArgs<R, S> &a, size_t smem, cudaStream_t s) {
-    cudaError_t e = cudaFuncSetAttribute(small_kernel<R, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = allow_smem<small_kernel<R, S>>();
     if (e != cudaSuccess) return e;
     small_kernel<R, S><<<unsigned(a.batch), small_threads(a.n), smem, s>>>(a);
     return cudaGetLastError();
