@@ -6,12 +6,16 @@ import threading
 
 import numpy as np
 
+from ..core import gates as G
+
 
 class KeptCircuits:
     """Rewritten forms of the last few circuits, with the programs lowered for them.
 
     Circuits are compared by content (their gates pickled: 0.15 ms for 56 gates), so a gate that was
-    changed in place is seen.  Safe with several threads; a copy starts empty."""
+    changed in place is seen.  What is kept is made from gates of its own, so that a later change of the caller's
+    gates does not reach it.  Circuits with gates of a caller's class or with matrices from a caller's function
+    are rewritten every time: a pickle names those only.  Safe with several threads; a copy starts empty."""
 
     LIMIT = 8
 
@@ -19,16 +23,23 @@ class KeptCircuits:
         self._lock = threading.Lock()
         self._items = {}
 
+    @staticmethod
+    def _by_content(gate):
+        return type(gate).__module__ == G.__name__ and not isinstance(gate, G.ParamNonHerm)
+
     def get(self, circ, rewrite):
-        """``rewrite(circ)``, or what it returned for the same gates."""
+        """``rewrite`` of the gates of ``circ`` (a list), or what it returned for the same gates."""
+        gates = list(circ)
+        if not all(map(self._by_content, gates)):
+            return rewrite(gates)
         try:
-            key = pickle.dumps(list(circ), -1)
+            key = pickle.dumps(gates, -1)
         except Exception:  # pylint: disable=broad-except
-            return rewrite(circ)   # gates that cannot be pickled (generators of custom gates)
+            return rewrite(gates)
         with self._lock:
             kept = self._items.pop(key, None)
         if kept is None:
-            kept = rewrite(circ)
+            kept = rewrite(pickle.loads(key))
         with self._lock:
             self._items[key] = kept   # the most recent one last
             while len(self._items) > self.LIMIT:
