@@ -163,6 +163,10 @@ MQB_API int mqb_program_grad_passes(mqb_program *prog, int n_hams, int *n_passes
 MQB_API int mqb_jit_check(int n_qubits, int precision, const mqb_gate_desc *gates, int n_gates,
                           const double *const_matrices, int64_t n_const_entries, int tile_bits, int n_hams,
                           int *n_kernels);
+/* Host-only: the most dynamic shared memory (bytes) that a generated kernel of the circuit's schedule asks for (at
+ * most 227 KB); the schedule of a gradient with n_hams Hamiltonians, or of a circuit's application (n_hams = 0). */
+MQB_API int mqb_jit_smem(int n_qubits, int precision, const mqb_gate_desc *gates, int n_gates,
+                         const double *const_matrices, int64_t n_const_entries, int n_hams, int64_t *bytes);
 
 /* Workspace (bytes) that mqb_apply needs for `batch` samples. */
 MQB_API int mqb_apply_workspace_size(const mqb_program *prog, int64_t batch, size_t *bytes);

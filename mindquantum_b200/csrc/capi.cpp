@@ -274,19 +274,21 @@ static const std::vector<const void *> *jit_backward(const mqb_program &p, Sched
 // Matrix-table entries a pass may hold so that the tile ring of its generated kernel (two groups, each with
 // its own table and gradient slots) keeps three buffers in 227 KB, or two where three leave less than 8 KB
 // for a table.  n_hams = 0: a forward schedule.
-static PassLimits pass_limits(const mqb_program &p, int K, int reg_bits, int n_hams) {
-    const int64_t buf = (int64_t(1) << K) * int64_t(p.elem()) * (1 + n_hams);
+static PassLimits pass_limits(int precision, int K, int reg_bits, int n_hams, bool use_jit) {
+    const int64_t eb = precision == MQB_PREC_C64 ? 8 : 16;
+    const int64_t buf = (int64_t(1) << K) * eb * (1 + n_hams);
     const int64_t warps = int64_t(1) << std::max(0, K - reg_bits - 5);
     const int64_t slots = n_hams ? warps * (kMaxPassSlots * n_hams * int64_t(sizeof(double)) + 512) : 0;
-    auto table = [&](int buffers) { return ((int64_t(227) << 10) - 256 - buffers * buf) / 2 - slots; };
+    // (multiples of 16, as the tables are laid out)
+    auto table = [&](int buffers) { return (((int64_t(227) << 10) - kJitFixedSmem - buffers * buf) / 2 - slots) & ~int64_t(15); };
     const int64_t bytes = table(3) >= 8192 ? table(3) : table(2);
     PassLimits lim;
-    lim.max_entries = int(std::max<int64_t>(bytes, 4096) / int64_t(p.elem()));
+    lim.max_entries = int(std::max<int64_t>(bytes, 4096) / eb);
     lim.derivatives = n_hams > 0;
     // Searched sets reorder gates, which in complex64 moves an expectation of 1e-2 by 1e-5 of itself; it pays
     // where passes cost (generated kernels) and is free of that in complex128 (16 qubits x 8 layers: 7 -> 4
     // passes, 0.67 -> 0.60 ms), but the precompiled complex64 kernels of smaller registers gain little.
-    lim.search = p.use_jit() || p.precision == MQB_PREC_C128;
+    lim.search = use_jit || precision == MQB_PREC_C128;
     return lim;
 }
 
@@ -350,7 +352,8 @@ static std::unique_ptr<SchedDev> make_sched(const mqb_program &p, int K, bool fu
     // state before its pass, and no gate with a gradient shares that pass
     for (size_t k = 0; n_hams > 0 && k < apart.size(); ++k)
         if (p.descs[k].gate_id == GID_MATRIX && !p.ops[k].unitary) apart[k] = 1;
-    sd->s = build_schedule(p.n, K, contiguity_bits(p.precision), p.ops, fuse, &apart, pass_limits(p, K, reg_bits, n_hams));
+    sd->s = build_schedule(p.n, K, contiguity_bits(p.precision), p.ops, fuse, &apart,
+                           pass_limits(p.precision, K, reg_bits, n_hams, p.use_jit()));
     build_stages(sd->s, p.ops, reg_bits, p.precision, false);
     build_stages(sd->s, p.ops, p.use_jit() ? jit_fwd_reg_bits(p.precision) : fwd_reg_bits(p.precision), p.precision, true);
     sd->s.d_pass_ops = upload(sd->s.pass_ops);
@@ -1165,29 +1168,55 @@ int mqb_plan_schedule(int n_qubits, int precision, const mqb_gate_desc *gates, i
     });
 }
 
+// The schedule of a gate table for generated kernels, on the host alone; n_hams = 0: a forward schedule.
+static Schedule host_jit_schedule(int n_qubits, int precision, const mqb_gate_desc *gates, int n_gates,
+                                  const double *const_matrices, int64_t n_const_entries, int tile_bits, int n_hams,
+                                  std::vector<DevOp> &ops) {
+    if (n_qubits < 1 || n_qubits > 40) fail(MQB_ERR_INVALID, "n_qubits must be in [1, 40]");
+    if (precision != MQB_PREC_C64 && precision != MQB_PREC_C128) fail(MQB_ERR_INVALID, "unknown precision");
+    if (n_hams < 0 || n_hams > 4) fail(MQB_ERR_INVALID, "invalid argument");
+    int slots = 0;
+    for (int k = 0; k < n_gates; ++k) {
+        DevOp op = basic_op(gates[k], k, n_qubits, nullptr, 0, 0, const_matrices, n_const_entries);
+        if (op.grad_mask) {
+            op.slot0 = slots;
+            for (int a = 0; a < op.n_angles; ++a) slots += (op.grad_mask >> a) & 1;
+        }
+        ops.push_back(op);
+    }
+    const int rb = n_hams ? bwd_reg_bits(precision, n_hams) : jit_fwd_reg_bits(precision);
+    int K = std::min(n_qubits, rb + 8);
+    if (tile_bits > 0) K = std::min(n_qubits, std::max(rb + 5, tile_bits));
+    Schedule s = build_schedule(n_qubits, K, contiguity_bits(precision), ops, K >= rb + 5, nullptr,
+                                pass_limits(precision, K, rb, n_hams, true));
+    build_stages(s, ops, rb, precision, false);
+    build_stages(s, ops, jit_fwd_reg_bits(precision), precision, true);
+    return s;
+}
+
 int mqb_jit_check(int n_qubits, int precision, const mqb_gate_desc *gates, int n_gates, const double *const_matrices,
                   int64_t n_const_entries, int tile_bits, int n_hams, int *n_kernels) {
     return guarded([&] {
-        if (n_qubits < 1 || n_qubits > 40) fail(MQB_ERR_INVALID, "n_qubits must be in [1, 40]");
-        if (precision != MQB_PREC_C64 && precision != MQB_PREC_C128) fail(MQB_ERR_INVALID, "unknown precision");
-        if (n_hams < 0 || n_hams > 4 || !n_kernels) fail(MQB_ERR_INVALID, "invalid argument");
+        if (!n_kernels) fail(MQB_ERR_INVALID, "invalid argument");
         std::vector<DevOp> ops;
-        int slots = 0;
-        for (int k = 0; k < n_gates; ++k) {
-            DevOp op = basic_op(gates[k], k, n_qubits, nullptr, 0, 0, const_matrices, n_const_entries);
-            if (op.grad_mask) {
-                op.slot0 = slots;
-                for (int a = 0; a < op.n_angles; ++a) slots += (op.grad_mask >> a) & 1;
-            }
-            ops.push_back(op);
-        }
-        const int rb = n_hams ? bwd_reg_bits(precision, n_hams) : jit_fwd_reg_bits(precision);
-        int K = std::min(n_qubits, rb + 8);
-        if (tile_bits > 0) K = std::min(n_qubits, std::max(rb + 5, tile_bits));
-        Schedule s = build_schedule(n_qubits, K, contiguity_bits(precision), ops, K >= rb + 5);
-        build_stages(s, ops, rb, precision, false);
-        build_stages(s, ops, jit_fwd_reg_bits(precision), precision, true);
+        const Schedule s = host_jit_schedule(n_qubits, precision, gates, n_gates, const_matrices, n_const_entries, tile_bits, n_hams, ops);
         *n_kernels = jit_compile_check(s, precision, n_hams, ops);
+    });
+}
+
+int mqb_jit_smem(int n_qubits, int precision, const mqb_gate_desc *gates, int n_gates, const double *const_matrices,
+                 int64_t n_const_entries, int n_hams, int64_t *bytes) {
+    return guarded([&] {
+        if (!bytes) fail(MQB_ERR_INVALID, "invalid argument");
+        std::vector<DevOp> ops;
+        const Schedule s = host_jit_schedule(n_qubits, precision, gates, n_gates, const_matrices, n_const_entries, 0, n_hams, ops);
+        size_t most = 0;
+        for (const Pass &ps : s.passes) {
+            if (!ps.fused) continue;
+            most = std::max(most, jit_forward_smem(ps, precision));
+            if (n_hams > 0) most = std::max(most, jit_backward_smem(ps, precision, n_hams));
+        }
+        *bytes = int64_t(most);
     });
 }
 

@@ -915,19 +915,23 @@ int fwd_groups(const Pass &p, int precision) {
     return std::min(max_groups(nt), env_int("MQB_PIPE_FWD_GROUPS", precision == MQB_PREC_C64 ? 1 : 2, 1, 15));
 }
 
-int fwd_buffers(const Pass &p, int precision) {
-    return std::max(fwd_groups(p, precision), env_int("MQB_PIPE_FWD_BUFFERS", precision == MQB_PREC_C64 ? 2 : 3, 1, 8));
-}
-
-// The ring's mbarriers and tickets, and the pass norm of each group.
-constexpr size_t kRingBytes = 8 * 16 + 8 * 16;
 constexpr size_t kSplitBytes = 16;   // sizeof(pipe::Split)
 
-size_t fwd_smem(const Pass &p, int precision) {
+size_t fwd_smem_of(const Pass &p, int precision, int buffers) {
     const size_t eb = elem_bytes(precision);
-    return size_t(fwd_buffers(p, precision)) * ((size_t(1) << p.K) * eb) +
-           size_t(fwd_groups(p, precision)) * (a16(size_t(p.f_mtab_entries) * eb) + size_t(p.f_run_entries) * kSplitBytes) + kRingBytes;
+    return size_t(buffers) * ((size_t(1) << p.K) * eb) +
+           size_t(fwd_groups(p, precision)) * (a16(size_t(p.f_mtab_entries) * eb) + size_t(p.f_run_entries) * kSplitBytes) + size_t(kJitFixedSmem);
 }
+
+// Buffers of the forward ring: as many of the wanted number as fit in 227 KB, at least one per group.
+int fwd_buffers(const Pass &p, int precision) {
+    const int G = fwd_groups(p, precision);
+    int nb = std::max(G, env_int("MQB_PIPE_FWD_BUFFERS", precision == MQB_PREC_C64 ? 2 : 3, 1, 8));
+    while (nb > G && fwd_smem_of(p, precision, nb) > size_t(227) << 10) --nb;
+    return nb;
+}
+
+size_t fwd_smem(const Pass &p, int precision) { return fwd_smem_of(p, precision, fwd_buffers(p, precision)); }
 
 int bwd_groups(const Pass &p) {
     const int nt = 1 << (p.K - p.reg_bits);
@@ -940,7 +944,7 @@ size_t bwd_fixed_smem(const Pass &p, int precision, int n_hams, int scratch, int
     return size_t(bwd_groups(p)) *
                (a16(size_t(p.mtab_entries) * eb) + a16(size_t(nw) * std::max(1, p.n_slots) * n_hams * sizeof(double)) +
                 size_t(nw) * size_t(scratch) + a16(size_t(runs) * eb)) +
-           kRingBytes;
+           size_t(kJitFixedSmem);
 }
 
 // Buffers of the adjoint ring: G + 1 where they fit in 227 KB, else as many as fit (at least G); 0: fewer than

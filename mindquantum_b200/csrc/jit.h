@@ -20,6 +20,9 @@ std::vector<const void *> jit_forward_kernels(const Schedule &s, int precision, 
 std::vector<const void *> jit_backward_kernels(const Schedule &s, int precision, int n_hams,
                                                const std::vector<DevOp> &ops);
 
+// Dynamic shared memory of a pass's kernels.  Besides the tile ring and each group's matrix table (and gradient rows, or
+// tables of runs) it holds kJitFixedSmem bytes: mbarriers and tickets of up to 8 buffers, and 16 pass norms.
+constexpr int kJitFixedSmem = 8 * 16 + 8 * 16;
 size_t jit_forward_smem(const Pass &p, int precision);
 size_t jit_backward_smem(const Pass &p, int precision, int n_hams);
 

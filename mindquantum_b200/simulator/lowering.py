@@ -203,21 +203,35 @@ def plan_schedule(circuit, n_qubits, precision, tile_bits=0, fuse=True):
     return order[:n], pass_of[:n], qmask[:k], fused[:k]
 
 
+def _gate_table(circuit):
+    """Gate records and constant matrices of ``circuit`` as the leading arguments of the host-only C calls."""
+    descs, _, pool, _, _ = lower_circuit(circuit, circuit.params_name)
+    gate_arr = (N.GateDesc * max(1, len(descs)))(*descs)
+    pool_arr = np.concatenate(pool) if pool else np.zeros(1, dtype=np.complex128)
+    pool_f = np.ascontiguousarray(pool_arr.astype(np.complex128)).view(np.float64)
+    return gate_arr, len(descs), pool_f, pool_arr.size
+
+
 def jit_check(circuit, n_qubits, precision, tile_bits=0, n_hams=0):
     """Generate and compile (NVRTC, no GPU needed) the pass kernels of ``circuit``.
 
     Forward kernels, plus the backward kernels for ``n_hams`` Hamiltonians when n_hams > 0.
     Returns the number of distinct kernels; raises with the compiler log on failure.
     """
-    descs, _, pool, _, _ = lower_circuit(circuit, circuit.params_name)
-    n = len(descs)
-    gate_arr = (N.GateDesc * max(1, n))(*descs)
-    pool_arr = np.concatenate(pool) if pool else np.zeros(1, dtype=np.complex128)
-    pool_f = np.ascontiguousarray(pool_arr.astype(np.complex128)).view(np.float64)
+    gates, n, pool, n_pool = _gate_table(circuit)
     count = ctypes.c_int()
-    N.call('mqb_jit_check', n_qubits, precision, gate_arr, n, pool_f.ctypes.data_as(ctypes.c_void_p), pool_arr.size,
+    N.call('mqb_jit_check', n_qubits, precision, gates, n, pool.ctypes.data_as(ctypes.c_void_p), n_pool,
            tile_bits, n_hams, ctypes.byref(count))
     return count.value
+
+
+def jit_smem(circuit, n_qubits, precision, n_hams=0):
+    """The most shared memory (bytes) that a generated pass kernel of ``circuit`` asks for (host only)."""
+    gates, n, pool, n_pool = _gate_table(circuit)
+    out = ctypes.c_int64()
+    N.call('mqb_jit_smem', n_qubits, precision, gates, n, pool.ctypes.data_as(ctypes.c_void_p), n_pool, n_hams,
+           ctypes.byref(out))
+    return out.value
 
 
 def lowered(circuit, n_qubits, precision, param_names, grad_names=None, fuse=True, tile_bits=0, jit=None):
