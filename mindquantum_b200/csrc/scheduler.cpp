@@ -13,7 +13,6 @@
 // of several candidates that takes the most gates (choose_set).
 #include <algorithm>
 #include <cstdlib>
-#include <iterator>
 #include <stdexcept>
 
 #include "mqb_internal.h"
@@ -97,17 +96,35 @@ struct ScanLimits {
     bool apart = false;              // the kind of items the set is for
 };
 
-// The items of `left` (indices, in program order) that can run together when the set is Q, which
+// The items that no group has taken yet, in program order: each one's successor (the number of items ends the list).
+struct Left {
+    int head = 0;
+    std::vector<int> next;
+
+    explicit Left(size_t n) : next(n) {
+        for (size_t i = 0; i < n; ++i) next[i] = int(i) + 1;
+    }
+    bool empty() const { return head == int(next.size()); }
+    void remove(const std::vector<int> &members) {   // (ascending)
+        int *at = &head;
+        for (int m : members) {
+            while (*at != m) at = &next[size_t(*at)];
+            *at = next[size_t(m)];
+        }
+    }
+};
+
+// The items of `left` that can run together when the set is Q, which
 // grows up to K qubits as the items ask for them when `grow`.  An item that cannot join blocks the
 // qubits it touches for the rest of the scan.  Returns how many join; `members` may be null; `wanted`
 // (optional) gets the qubits outside Q that kept an otherwise free item out.
-int scan_items(const std::vector<ScanItem> &items, const std::vector<int> &left, const ScanLimits &lim, uint64_t &Q,
+int scan_items(const std::vector<ScanItem> &items, const Left &left, const ScanLimits &lim, uint64_t &Q,
                bool grow, std::vector<int> *members, uint64_t *wanted = nullptr) {
     uint64_t blocked = 0;
     if (wanted) *wanted = 0;
     int n_items = 0, n_slots = 0, n_entries = 0;
-    for (int i : left) {
-        const ScanItem &it = items[i];
+    for (int i = left.head; i < int(items.size()); i = left.next[size_t(i)]) {
+        const ScanItem &it = items[size_t(i)];
         if (n_items >= lim.max_items) break;
         const uint64_t need = it.dense & ~Q;
         if ((it.touch & blocked) || !it.fusable || it.apart != lim.apart || (need && (!grow || popc(Q | need) > lim.K)) ||
@@ -133,7 +150,7 @@ int scan_items(const std::vector<ScanItem> &items, const std::vector<int> &left,
 // neighbours outside it.  A window next to the qubits that earlier passes brought furthest lets a
 // wedge of many layers through (26 qubits x 12 layers of RY, RZ and a CNOT ladder, 12-qubit sets: 14
 // passes instead of 31).  Ties keep the program-order set.
-uint64_t choose_set(const std::vector<ScanItem> &items, const std::vector<int> &left, const ScanLimits &lim,
+uint64_t choose_set(const std::vector<ScanItem> &items, const Left &left, const ScanLimits &lim,
                     uint64_t Q0, int n, bool windows) {
     uint64_t best_q = Q0;
     int best = scan_items(items, left, lim, best_q, true, nullptr);
@@ -184,25 +201,22 @@ struct Cut {
 // Cut the items into groups, each group's set taken in program order or, with `search`, by choose_set.
 std::vector<Cut> cut_items(const std::vector<ScanItem> &items, ScanLimits lim, uint64_t Q0, int n, bool windows,
                            bool search) {
-    std::vector<int> left(items.size()), rest;
-    for (size_t i = 0; i < items.size(); ++i) left[i] = int(i);
+    Left left(items.size());
     std::vector<Cut> out;
     while (!left.empty()) {
         Cut c;
-        if (items[size_t(left.front())].fusable) {
+        if (items[size_t(left.head)].fusable) {
             c.set = Q0;
-            lim.apart = items[size_t(left.front())].apart;
+            lim.apart = items[size_t(left.head)].apart;
             if (search) c.set = choose_set(items, left, lim, Q0, n, windows);
             scan_items(items, left, lim, c.set, !search, &c.members);
         }
         if (c.members.empty()) {
             // not fusable, or too wide for the room next to Q0
             c.single = true;
-            c.members.push_back(left.front());
+            c.members.push_back(left.head);
         }
-        rest.clear();
-        std::set_difference(left.begin(), left.end(), c.members.begin(), c.members.end(), std::back_inserter(rest));
-        left.swap(rest);
+        left.remove(c.members);
         out.push_back(std::move(c));
     }
     return out;
@@ -247,7 +261,7 @@ Schedule build_schedule(int n, int K, int c, const std::vector<DevOp> &ops, bool
     lim.max_items = kMaxPassOps;
     lim.max_slots = kMaxPassSlots;
     lim.max_entries = limits.max_entries;
-    lim.all = all;
+    for (const ScanItem &it : items) lim.all |= it.touch;   // (a scan ends when they are blocked: idle qubits never are)
     for (const Cut &cut : best_cut(items, lim, (n <= K) ? all : ((uint64_t(1) << c) - 1), n, true, limits.search)) {
         const std::vector<int> &members = cut.members;
         if (cut.single) {
