@@ -209,6 +209,9 @@ struct SchedDev {
     }
 };
 
+// Programs of this many qubits run generated kernels by default.
+constexpr int kJitMinQubits = 18;
+
 struct mqb_program {
     int n = 0, precision = 0, n_params = 0, fuse = 1, tile_bits = 0, jit = 0;
     std::vector<DevOp> ops;
@@ -240,7 +243,7 @@ struct mqb_program {
     }
     size_t elem() const { return precision == MQB_PREC_C64 ? 8 : 16; }
     // generated pass kernels pay their compile time back from 2^18 amplitudes on
-    bool use_jit() const { return jit > 0 || (jit == 0 && n >= 18); }
+    bool use_jit() const { return jit > 0 || (jit == 0 && n >= kJitMinQubits); }
 };
 
 // Calls that promise to allocate nothing (mqb_apply_static) run the precompiled kernels only.
@@ -290,6 +293,13 @@ static PassLimits pass_limits(int precision, int K, int reg_bits, int n_hams, bo
     // passes, 0.67 -> 0.60 ms), but the precompiled complex64 kernels of smaller registers gain little.
     lim.search = use_jit || precision == MQB_PREC_C128;
     return lim;
+}
+
+// Tile size of the fused kernels: 2^RB registers x 2^8 threads, capped by the register size.
+static int tile_bits_of(int n, int tile_bits, int reg_bits) {
+    int K = reg_bits + 8;
+    if (tile_bits > 0) K = std::min(K, std::max(reg_bits + 5, tile_bits));
+    return std::min(K, n);
 }
 
 static int norm_stride(int passes) { return std::max(1, int(std::ceil(std::sqrt(double(passes))))); }
@@ -368,20 +378,13 @@ static std::unique_ptr<SchedDev> make_sched(const mqb_program &p, int K, bool fu
     return sd;
 }
 
-// Tile size of the fused kernels: 2^RB registers x 2^8 threads, capped by the register size.
-static int tile_bits_for(const mqb_program &p, int reg_bits) {
-    int K = reg_bits + 8;
-    if (p.tile_bits > 0) K = std::min(K, std::max(reg_bits + 5, p.tile_bits));
-    return std::min(K, p.n);
-}
-
 static SchedDev &grad_schedule(mqb_program &p, int n_hams) {
     const bool fused = p.fuse && n_hams <= 4;
     const int key = fused ? n_hams : 0;
     auto it = p.grad_sched.find(key);
     if (it != p.grad_sched.end()) return *it->second;
     const int rb = bwd_reg_bits(p.precision, n_hams);
-    auto sd = make_sched(p, fused ? tile_bits_for(p, rb) : p.n, fused, rb, n_hams);
+    auto sd = make_sched(p, fused ? tile_bits_of(p.n, p.tile_bits, rb) : p.n, fused, rb, n_hams);
     SchedDev &ref = *sd;
     p.grad_sched[key] = std::move(sd);
     return ref;
@@ -1127,7 +1130,7 @@ int mqb_program_create(int n_qubits, int precision, const mqb_gate_desc *gates, 
         p->d_csr_slot = upload(slot);
         p->d_csr_coeff = upload(coeff);
         const int rb = p->use_jit() ? jit_fwd_reg_bits(precision) : fwd_reg_bits(precision);
-        p->apply_sched = make_sched(*p, tile_bits_for(*p, rb), p->fuse != 0, rb, 0);
+        p->apply_sched = make_sched(*p, tile_bits_of(p->n, p->tile_bits, rb), p->fuse != 0, rb, 0);
         *out = p.release();
     });
 }
@@ -1140,11 +1143,13 @@ int mqb_plan_schedule(int n_qubits, int precision, const mqb_gate_desc *gates, i
         std::vector<DevOp> ops;
         for (int k = 0; k < n_gates; ++k)
             ops.push_back(basic_op(gates[k], k, n_qubits, nullptr, 0, 0, const_matrices, n_const_entries));
-        // the register bits mqb_program_create takes by default (generated kernels from 18 qubits on)
-        const int rb = n_qubits >= 18 && tile_bits == 0 ? jit_fwd_reg_bits(precision) : fwd_reg_bits(precision);
-        int K = std::min(n_qubits, rb + 8);
-        if (tile_bits > 0) K = std::min(n_qubits, std::max(rb + 5, tile_bits));
-        Schedule s = build_schedule(n_qubits, K, contiguity_bits(precision), ops, fuse != 0 && K >= rb + 5);
+        // as mqb_program_create lays the circuit's application out by default
+        std::vector<char> apart(ops.size());
+        for (int k = 0; k < n_gates; ++k) apart[size_t(k)] = (gates[k].flags & MQB_GATE_NONUNITARY) != 0;
+        const bool use_jit = n_qubits >= kJitMinQubits;
+        const int rb = use_jit ? jit_fwd_reg_bits(precision) : fwd_reg_bits(precision), K = tile_bits_of(n_qubits, tile_bits, rb);
+        Schedule s = build_schedule(n_qubits, K, contiguity_bits(precision), ops, fuse != 0 && K >= rb + 5, &apart,
+                                    pass_limits(precision, K, rb, 0, use_jit));
         build_stages(s, ops, rb, precision, true);
         int pos = 0;
         for (size_t pi = 0; pi < s.passes.size(); ++pi) {
@@ -1185,8 +1190,7 @@ static Schedule host_jit_schedule(int n_qubits, int precision, const mqb_gate_de
         ops.push_back(op);
     }
     const int rb = n_hams ? bwd_reg_bits(precision, n_hams) : jit_fwd_reg_bits(precision);
-    int K = std::min(n_qubits, rb + 8);
-    if (tile_bits > 0) K = std::min(n_qubits, std::max(rb + 5, tile_bits));
+    const int K = tile_bits_of(n_qubits, tile_bits, rb);
     Schedule s = build_schedule(n_qubits, K, contiguity_bits(precision), ops, K >= rb + 5, nullptr,
                                 pass_limits(precision, K, rb, n_hams, true));
     build_stages(s, ops, rb, precision, false);
