@@ -231,6 +231,7 @@ struct mqb_program {
     bool nonunitary = false;
     std::unique_ptr<SchedDev> apply_sched;
     std::map<int, std::unique_ptr<SchedDev>> grad_sched;   // by number of Hamiltonians
+    std::mutex grad_mu;                                    // ... made on first use, by whichever thread
     ~mqb_program() {
         cudaFree(d_ops);
         cudaFree(d_descs);
@@ -381,6 +382,7 @@ static std::unique_ptr<SchedDev> make_sched(const mqb_program &p, int K, bool fu
 static SchedDev &grad_schedule(mqb_program &p, int n_hams) {
     const bool fused = p.fuse && n_hams <= 4;
     const int key = fused ? n_hams : 0;
+    std::lock_guard<std::mutex> lk(p.grad_mu);
     auto it = p.grad_sched.find(key);
     if (it != p.grad_sched.end()) return *it->second;
     const int rb = bwd_reg_bits(p.precision, n_hams);

@@ -50,3 +50,22 @@ def test_launch_limits_of_two_circuits(n, layers):
     for got, (f, g) in zip(_in_threads(jobs, 300), expected):
         for f1, g1 in got:
             assert np.allclose(f1, f, atol=1e-12) and np.allclose(g1, g, atol=1e-11)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('backend,n', [('mqvector_b200', 9), ('mqmatrix_b200', 4)])
+def test_first_gradients_of_one_circuit(backend, n):
+    """Threads that evaluate one circuit share its program, whose gradient schedules are made on first use."""
+    for seed in range(10):
+        circ = hea_circuit(n, 1 + seed % 3)
+        hams = [Hamiltonian(QubitOperator(f'Z{q}')) for q in range(4)]
+        p = np.random.default_rng(seed).uniform(0, 2 * np.pi, size=len(circ.params_name))
+        if backend == 'mqmatrix_b200':   # one simulator, whose doubled circuit is kept for all calls
+            sims = [Simulator(backend, n, dtype=complex128)] * 4
+        else:
+            sims = [Simulator(backend, n, dtype=complex128) for _ in range(4)]
+        jobs = [lambda op=sim.get_expectation_with_grad(hams[:k + 1], circ): op(p) for k, sim in enumerate(sims)]
+        got = _in_threads(jobs, 1)
+        for k, ((f, g),) in enumerate(got):
+            f1, g1 = Simulator(backend, n, dtype=complex128).get_expectation_with_grad(hams[:k + 1], hea_circuit(n, 1 + seed % 3))(p)
+            assert np.allclose(f, f1, atol=1e-11) and np.allclose(g, g1, atol=1e-11)
