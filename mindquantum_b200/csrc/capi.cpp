@@ -309,10 +309,20 @@ static int norm_stride(int passes) { return std::max(1, int(std::ceil(std::sqrt(
 // against 7 and more): at 10 qubits it and the tile kernels both hide behind the host's 260 us per call, at 11
 // one sample with 4 Hamiltonians takes 409 us here and 400 there, at 12 724 against 505.
 constexpr int kSmallMaxQubits = 10;
-// Registers up to this size run here at any batch, larger ones up to two samples per SM: with 1024
-// samples, 8 qubits take 376 (complex64, 4 Hamiltonians) and 269 us (complex128, one) against 341 and 288
-// of the tile kernels, 9 qubits 475 against 321, 10 qubits 1030 against 429.
-constexpr int kSmallAnyBatchQubits = 8;
+// Where tile passes could run a register too, it runs here up to this many samples: one per SM at 10 qubits and twice as
+// many per qubit less, as a block's work and its shared memory go, and twice that for a complex64 state alone.  A
+// 3-layer ansatz, here / tile kernels, us.  Gradients:
+//   complex64, 2 Hamiltonians:  8 qubits, 592 samples 157 / 172, 888 samples 277 / 184; 9 qubits, 296 samples 176 / 196;
+//                               10 qubits, 148 samples 198 / 221, 296 samples 384 / 235
+//   complex64, 4 Hamiltonians:  592 samples 212 / 235, 888 375 / 273; 236 / 280; 266 / 311, 519 / 354
+//   complex128, 2 Hamiltonians: 7 qubits, 1184 samples 143 / 156, 1480 251 / 182; 8 qubits, 592 155 / 159, 888 272 / 179;
+//                               9 qubits, 296 173 / 192; 10 qubits, 148 196 / 191, 296 379 / 221
+// Applications: complex64, 10 qubits, 148 samples 45 / 87, 296 81 / 91; complex128, 9 qubits, 296 49 / 78; 10 qubits, 148
+// 50 / 66, 296 93 / 70.
+static int64_t small_max_batch(int n, int precision, bool gradient) {
+    const int64_t sm = sm_count_cached();
+    return (gradient || precision == MQB_PREC_C128 ? sm : 2 * sm) << (kSmallMaxQubits - n);
+}
 
 // The block-per-sample kernel's gate list, in the schedule's execution order, when it can run the
 // program: gates of at most two targets, everything in one block's shared memory.  Callers that force a kernel family (jit, tile_bits, fuse) get that one.
@@ -478,10 +488,10 @@ static void run_matgen(const mqb_program &p, const double *params, int64_t param
 // Whether a call runs the block-per-sample kernel: the schedule has it, and the tile kernels either cannot
 // fuse this register or are not the faster ones at this batch, or undo gates that they should not (a custom gate, whose
 // matrices the caller makes: its evaluation on the host takes longer than either kernel).
-static bool runs_small(const mqb_program &p, const SchedDev &sd, int64_t batch) {
+static bool runs_small(const mqb_program &p, const SchedDev &sd, int64_t batch, bool gradient) {
     if (!sd.small_smem) return false;
     const bool tiles = std::any_of(sd.s.passes.begin(), sd.s.passes.end(), [](const Pass &ps) { return ps.fused != 0; });
-    return !tiles || sd.small_saved || p.n <= kSmallAnyBatchQubits || batch <= 2 * int64_t(sm_count_cached());
+    return !tiles || sd.small_saved || batch <= small_max_batch(p.n, p.precision, gradient);
 }
 
 template <typename R, typename S>
@@ -507,7 +517,7 @@ static void apply_impl(mqb_program &p, void *states, int64_t batch, const double
     cplx<R> *mats = static_cast<cplx<R> *>(ws);
     cplx<R> *s = static_cast<cplx<R> *>(states);
     SchedDev &sd = *p.apply_sched;
-    if (runs_small(p, sd, batch)) {
+    if (runs_small(p, sd, batch, false)) {
         run_matgen<R>(p, params, param_stride, custom, batch, mats, st);
         SmallArgs<R, R> a = small_args<R, R>(p, sd, mats, p.d_cpool, batch);
         a.src = s;
@@ -693,7 +703,7 @@ static void grad_impl(mqb_program &p, const mqb_hamiltonian *const *hams, int n_
     const int sm = sm_count_cached();
     const V *cpool = static_cast<const V *>(p.d_cpool);
 
-    if (runs_small(p, sd, batch) && std::none_of(hams, hams + (lam_in ? 0 : n_hams), [](const mqb_hamiltonian *h) { return h->csr; })) {
+    if (runs_small(p, sd, batch, true) && std::none_of(hams, hams + (lam_in ? 0 : n_hams), [](const mqb_hamiltonian *h) { return h->csr; })) {
         cplx<double> *wide = reinterpret_cast<cplx<double> *>(base);   // FP64 whatever the caller's precision
         run_matgen<double>(p, params, param_stride, custom, batch, wide, st);
         SmallArgs<double, R> a = small_args<double, R>(p, sd, wide, p.d_cpool64, batch);
