@@ -211,6 +211,12 @@ struct SchedDev {
 
 // Programs of this many qubits run generated kernels by default.
 constexpr int kJitMinQubits = 18;
+// mqb_apply_static runs precompiled passes, which like larger tiles than the generated ones where the tiles are many, so that
+// complex64 programs of this many qubits keep a schedule for it (it may allocate nothing later).  A 6-layer ansatz and 200
+// mixed gates, 2^12-amplitude tiles with searched sets / 2^13 in program order, us: 20 qubits 261 / 313 and 222 / 320; 22
+// qubits 971 / 982 and 750 / 738; 23 qubits 1762 / 1965 and 1271 / 1327; 24 qubits 3682 / 3637 and 2572 / 2444; 26 qubits 15527 /
+// 15472 and 9417 / 8924.
+constexpr int kStaticSchedQubits = 24;
 
 struct mqb_program {
     int n = 0, precision = 0, n_params = 0, fuse = 1, tile_bits = 0, jit = 0;
@@ -230,6 +236,7 @@ struct mqb_program {
     std::vector<char> apart;   // per op: MQB_GATE_NONUNITARY
     bool nonunitary = false;
     std::unique_ptr<SchedDev> apply_sched;
+    std::unique_ptr<SchedDev> static_sched;                // mqb_apply_static's own (kStaticSchedQubits), else apply_sched
     std::map<int, std::unique_ptr<SchedDev>> grad_sched;   // by number of Hamiltonians
     std::mutex grad_mu;                                    // ... made on first use, by whichever thread
     ~mqb_program() {
@@ -363,7 +370,8 @@ static void plan_small(const mqb_program &p, SchedDev &sd, int n_hams) {
     sd.small_smem = smem;
 }
 
-static std::unique_ptr<SchedDev> make_sched(const mqb_program &p, int K, bool fuse, int reg_bits, int n_hams) {
+// `generated`: laid out for generated kernels.
+static std::unique_ptr<SchedDev> make_sched(const mqb_program &p, int K, bool fuse, int reg_bits, int n_hams, bool generated) {
     auto sd = std::make_unique<SchedDev>();
     // the register kernels need 2^5..2^8 threads of 2^reg_bits amplitudes: smaller registers use
     // the per-gate kernels
@@ -374,9 +382,9 @@ static std::unique_ptr<SchedDev> make_sched(const mqb_program &p, int K, bool fu
     for (size_t k = 0; n_hams > 0 && k < apart.size(); ++k)
         if (p.descs[k].gate_id == GID_MATRIX && !p.ops[k].unitary) apart[k] = 1;
     sd->s = build_schedule(p.n, K, contiguity_bits(p.precision), p.ops, fuse, &apart,
-                           pass_limits(p.precision, K, reg_bits, n_hams, p.use_jit()));
+                           pass_limits(p.precision, K, reg_bits, n_hams, generated));
     build_stages(sd->s, p.ops, reg_bits, p.precision, false);
-    build_stages(sd->s, p.ops, p.use_jit() ? jit_fwd_reg_bits(p.precision) : fwd_reg_bits(p.precision), p.precision, true);
+    build_stages(sd->s, p.ops, generated ? jit_fwd_reg_bits(p.precision) : fwd_reg_bits(p.precision), p.precision, true);
     sd->s.d_pass_ops = upload(sd->s.pass_ops);
     sd->s.d_slot_map = upload(sd->s.slot_map);
     sd->s.d_stages = upload(sd->s.stages);
@@ -396,7 +404,7 @@ static SchedDev &grad_schedule(mqb_program &p, int n_hams) {
     auto it = p.grad_sched.find(key);
     if (it != p.grad_sched.end()) return *it->second;
     const int rb = bwd_reg_bits(p.precision, n_hams);
-    auto sd = make_sched(p, fused ? tile_bits_of(p.n, p.tile_bits, rb) : p.n, fused, rb, n_hams);
+    auto sd = make_sched(p, fused ? tile_bits_of(p.n, p.tile_bits, rb) : p.n, fused, rb, n_hams, p.use_jit());
     SchedDev &ref = *sd;
     p.grad_sched[key] = std::move(sd);
     return ref;
@@ -516,7 +524,7 @@ static void apply_impl(mqb_program &p, void *states, int64_t batch, const double
     if (p.per_sample && (ws == nullptr || ws_bytes < need)) fail(MQB_ERR_WORKSPACE, "workspace too small");
     cplx<R> *mats = static_cast<cplx<R> *>(ws);
     cplx<R> *s = static_cast<cplx<R> *>(states);
-    SchedDev &sd = *p.apply_sched;
+    SchedDev &sd = t_jit_blocked && p.static_sched ? *p.static_sched : *p.apply_sched;
     if (runs_small(p, sd, batch, false)) {
         run_matgen<R>(p, params, param_stride, custom, batch, mats, st);
         SmallArgs<R, R> a = small_args<R, R>(p, sd, mats, p.d_cpool, batch);
@@ -1142,7 +1150,11 @@ int mqb_program_create(int n_qubits, int precision, const mqb_gate_desc *gates, 
         p->d_csr_slot = upload(slot);
         p->d_csr_coeff = upload(coeff);
         const int rb = p->use_jit() ? jit_fwd_reg_bits(precision) : fwd_reg_bits(precision);
-        p->apply_sched = make_sched(*p, tile_bits_of(p->n, p->tile_bits, rb), p->fuse != 0, rb, 0);
+        p->apply_sched = make_sched(*p, tile_bits_of(p->n, p->tile_bits, rb), p->fuse != 0, rb, 0, p->use_jit());
+        if (p->use_jit() && precision == MQB_PREC_C64 && n_qubits >= kStaticSchedQubits) {
+            const int sb = fwd_reg_bits(precision);
+            p->static_sched = make_sched(*p, tile_bits_of(p->n, p->tile_bits, sb), p->fuse != 0, sb, 0, false);
+        }
         *out = p.release();
     });
 }
