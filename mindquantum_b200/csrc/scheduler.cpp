@@ -96,21 +96,26 @@ struct ScanLimits {
     bool apart = false;              // the kind of items the set is for
 };
 
-// The items that no group has taken yet, in program order: each one's successor (the number of items ends the list).
+// The items that no group has taken yet, in program order: list[head..).  Removing a group moves the kept items before its last
+// one up, so that it costs no more than the scan that found it; the scans, which are many, read an array.
 struct Left {
-    int head = 0;
-    std::vector<int> next;
+    std::vector<int> list;
+    size_t head = 0;
 
-    explicit Left(size_t n) : next(n) {
-        for (size_t i = 0; i < n; ++i) next[i] = int(i) + 1;
+    explicit Left(size_t n) : list(n) {
+        for (size_t i = 0; i < n; ++i) list[i] = int(i);
     }
-    bool empty() const { return head == int(next.size()); }
-    void remove(const std::vector<int> &members) {   // (ascending)
-        int *at = &head;
-        for (int m : members) {
-            while (*at != m) at = &next[size_t(*at)];
-            *at = next[size_t(m)];
+    bool empty() const { return head == list.size(); }
+    int front() const { return list[head]; }
+    void remove(const std::vector<int> &members) {   // (ascending, not empty)
+        size_t from = head, m = members.size();
+        while (list[from] != members.back()) ++from;
+        size_t to = from + 1;
+        for (size_t p = from + 1; p-- > head;) {
+            if (m > 0 && list[p] == members[m - 1]) --m;
+            else list[--to] = list[p];
         }
+        head = to;
     }
 };
 
@@ -123,7 +128,8 @@ int scan_items(const std::vector<ScanItem> &items, const Left &left, const ScanL
     uint64_t blocked = 0;
     if (wanted) *wanted = 0;
     int n_items = 0, n_slots = 0, n_entries = 0;
-    for (int i = left.head; i < int(items.size()); i = left.next[size_t(i)]) {
+    for (size_t p = left.head; p < left.list.size(); ++p) {
+        const int i = left.list[p];
         const ScanItem &it = items[size_t(i)];
         if (n_items >= lim.max_items) break;
         const uint64_t need = it.dense & ~Q;
@@ -205,16 +211,16 @@ std::vector<Cut> cut_items(const std::vector<ScanItem> &items, ScanLimits lim, u
     std::vector<Cut> out;
     while (!left.empty()) {
         Cut c;
-        if (items[size_t(left.head)].fusable) {
+        if (items[size_t(left.front())].fusable) {
             c.set = Q0;
-            lim.apart = items[size_t(left.head)].apart;
+            lim.apart = items[size_t(left.front())].apart;
             if (search) c.set = choose_set(items, left, lim, Q0, n, windows);
             scan_items(items, left, lim, c.set, !search, &c.members);
         }
         if (c.members.empty()) {
             // not fusable, or too wide for the room next to Q0
             c.single = true;
-            c.members.push_back(left.head);
+            c.members.push_back(left.front());
         }
         left.remove(c.members);
         out.push_back(std::move(c));
