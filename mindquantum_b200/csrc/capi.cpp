@@ -200,7 +200,6 @@ struct SchedDev {
         cudaFree(d_small);
         cudaFree(d_jmt);
         cudaFree(d_f_jmt);
-        cudaFree(s.d_pass_ops);
         cudaFree(s.d_slot_map);
         cudaFree(s.d_stages);
         cudaFree(s.d_stage_ops);
@@ -370,7 +369,7 @@ static void plan_small(const mqb_program &p, SchedDev &sd, int n_hams) {
     sd.small_smem = smem;
 }
 
-// `generated`: laid out for generated kernels.
+// `generated`: laid out for generated kernels.  Without Hamiltonians the schedule is for applications, forward passes alone.
 static std::unique_ptr<SchedDev> make_sched(const mqb_program &p, int K, bool fuse, int reg_bits, int n_hams, bool generated) {
     auto sd = std::make_unique<SchedDev>();
     // the register kernels need 2^5..2^8 threads of 2^reg_bits amplitudes: smaller registers use
@@ -383,16 +382,17 @@ static std::unique_ptr<SchedDev> make_sched(const mqb_program &p, int K, bool fu
         if (p.descs[k].gate_id == GID_MATRIX && !p.ops[k].unitary) apart[k] = 1;
     sd->s = build_schedule(p.n, K, contiguity_bits(p.precision), p.ops, fuse, &apart,
                            pass_limits(p.precision, K, reg_bits, n_hams, generated));
-    build_stages(sd->s, p.ops, reg_bits, p.precision, false);
     build_stages(sd->s, p.ops, generated ? jit_fwd_reg_bits(p.precision) : fwd_reg_bits(p.precision), p.precision, true);
-    sd->s.d_pass_ops = upload(sd->s.pass_ops);
-    sd->s.d_slot_map = upload(sd->s.slot_map);
-    sd->s.d_stages = upload(sd->s.stages);
-    sd->s.d_stage_ops = upload(sd->s.stage_ops);
     sd->s.d_f_stages = upload(sd->s.f_stages);
     sd->s.d_f_stage_ops = upload(sd->s.f_stage_ops);
-    sd->d_jmt = upload(jit_mtab(sd->s.stage_ops));
     sd->d_f_jmt = upload(jit_mtab(sd->s.f_stage_ops));
+    if (n_hams > 0) {
+        build_stages(sd->s, p.ops, reg_bits, p.precision, false);
+        sd->s.d_slot_map = upload(sd->s.slot_map);
+        sd->s.d_stages = upload(sd->s.stages);
+        sd->s.d_stage_ops = upload(sd->s.stage_ops);
+        sd->d_jmt = upload(jit_mtab(sd->s.stage_ops));
+    }
     plan_small(p, *sd, n_hams);
     return sd;
 }

@@ -156,8 +156,7 @@ struct Schedule {
     std::vector<StageOp> f_stage_ops;
     StageDesc *d_f_stages = nullptr;
     StageOp *d_f_stage_ops = nullptr;
-    PassOp *d_pass_ops = nullptr;   // device copies
-    int32_t *d_slot_map = nullptr;
+    int32_t *d_slot_map = nullptr;  // device copies
     StageDesc *d_stages = nullptr;
     StageOp *d_stage_ops = nullptr;
 };
