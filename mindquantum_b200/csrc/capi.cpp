@@ -299,6 +299,7 @@ static PassLimits pass_limits(int precision, int K, int reg_bits, int n_hams, bo
     // where passes cost (generated kernels) and is free of that in complex128 (16 qubits x 8 layers: 7 -> 4
     // passes, 0.67 -> 0.60 ms), but the precompiled complex64 kernels of smaller registers gain little.
     lim.search = use_jit || precision == MQB_PREC_C128;
+    lim.boxes = use_jit;
     return lim;
 }
 

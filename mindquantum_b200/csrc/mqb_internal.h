@@ -207,6 +207,7 @@ struct PassLimits {
     int max_entries = 1 << 30;   // complex entries of the pass's shared-memory matrix table
     bool derivatives = true;     // whether the table holds the gates' derivative matrices too
     bool search = true;          // search the sets (else program order)
+    bool boxes = true;           // tiles are moved by tensor copies, whose number depends on the set
 };
 
 // Builders (scheduler.cpp)

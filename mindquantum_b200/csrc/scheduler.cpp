@@ -94,7 +94,17 @@ struct ScanLimits {
     int max_items = 1 << 30, max_slots = 1 << 30, max_entries = 1 << 30;
     uint64_t all = 0;
     bool apart = false;              // the kind of items the set is for
+    bool boxes = false;              // sets are moved by tensor copies (box_cost)
 };
+
+// Time of a pass over the tiles of set Q against one that is moved whole.  A tensor copy takes the low run of consecutive
+// qubits and four more; each further run doubles the copies per tile.  Adjoint passes of some 40 gates on 30 qubits: 16.0
+// ms with 1 copy per tile, 17.1 with 2, 20.9 with 4, 25.9 with 8 and 39 with 16.
+double box_cost(uint64_t Q) {
+    static const double cost[] = {1.0, 1.07, 1.3, 1.6, 2.4, 4.0};
+    const int runs = popc(Q & ~(Q << 1));
+    return cost[std::min(5, std::max(0, runs - 5))];
+}
 
 // The items that no group has taken yet, in program order: list[head..).  Removing a group moves the kept items before its last
 // one up, so that it costs no more than the scan that found it; the scans, which are many, read an array.
@@ -149,9 +159,10 @@ int scan_items(const std::vector<ScanItem> &items, const Left &left, const ScanL
     return n_items;
 }
 
-// The set of at most K qubits, Q0 among them, under which the most items of `left` run together, out
-// of: the qubits in the order the items ask for them; every window of consecutive qubits above
-// Q0 (`windows`); and Q0 grown by the qubit that lets most items join, one at a time.  In a layered circuit a
+// The set of at most K qubits, Q0 among them, under which the most items of `left` run together (per time of the pass,
+// `lim.boxes`), out of: the qubits in the order the items ask for them; every window of consecutive qubits above
+// Q0 (`windows`); and Q0 grown by the qubit that lets most items join, one at a time, freely and (`lim.boxes`) without a
+// further run of qubits where that would double the copies per tile.  In a layered circuit a
 // set taken in program order is used for about two layers: the gates of later layers wait for
 // neighbours outside it.  A window next to the qubits that earlier passes brought furthest lets a
 // wedge of many layers through (26 qubits x 12 layers of RY, RZ and a CNOT ladder, 12-qubit sets: 14
@@ -159,11 +170,13 @@ int scan_items(const std::vector<ScanItem> &items, const Left &left, const ScanL
 uint64_t choose_set(const std::vector<ScanItem> &items, const Left &left, const ScanLimits &lim,
                     uint64_t Q0, int n, bool windows) {
     uint64_t best_q = Q0;
-    int best = scan_items(items, left, lim, best_q, true, nullptr);
+    const int plain = scan_items(items, left, lim, best_q, true, nullptr);
     if (n <= lim.K) return best_q;
+    auto rate = [&](uint64_t Q, int got) { return lim.boxes ? got / box_cost(Q) : double(got); };
+    double best = rate(best_q, plain);
     auto offer = [&](uint64_t Q, int got) {
-        if (got > best) {
-            best = got;
+        if (rate(Q, got) > best) {
+            best = rate(Q, got);
             best_q = Q;
         }
     };
@@ -175,25 +188,34 @@ uint64_t choose_set(const std::vector<ScanItem> &items, const Left &left, const 
             if (popc(Q) == lim.K) offer(Q, scan_items(items, left, lim, Q, false, nullptr));
         }
     }
-    uint64_t Q = Q0, wanted = 0;
-    int got = scan_items(items, left, lim, Q, false, nullptr, &wanted);
-    while (popc(Q) < lim.K && wanted) {   // only a wanted qubit lets more items join
-        int step_got = -1;
-        uint64_t step_q = Q, step_wanted = 0;
-        for (uint64_t rest = wanted; rest; rest &= rest - 1) {
-            uint64_t t = Q | (rest & ~(rest - 1)), w = 0;
-            const int g = scan_items(items, left, lim, t, false, nullptr, &w);
-            if (g > step_got) {
-                step_got = g;
-                step_q = t;
-                step_wanted = w;
+    for (int whole = 0; whole <= (lim.boxes ? 1 : 0); ++whole) {
+        uint64_t Q = Q0, wanted = 0;
+        int got = scan_items(items, left, lim, Q, false, nullptr, &wanted);
+        bool met = false;   // the second growth differs from the first
+        while (popc(Q) < lim.K && wanted) {   // only a wanted qubit lets more items join
+            int step_got = -1;
+            uint64_t step_q = Q, step_wanted = 0;
+            for (uint64_t rest = wanted; rest; rest &= rest - 1) {
+                uint64_t t = Q | (rest & ~(rest - 1)), w = 0;
+                if (whole && box_cost(t) > box_cost(Q)) {
+                    met = true;
+                    continue;
+                }
+                const int g = scan_items(items, left, lim, t, false, nullptr, &w);
+                if (g > step_got) {
+                    step_got = g;
+                    step_q = t;
+                    step_wanted = w;
+                }
             }
+            if (step_got < 0) break;
+            Q = step_q;
+            got = step_got;
+            wanted = step_wanted;
         }
-        Q = step_q;
-        got = step_got;
-        wanted = step_wanted;
+        if (!whole || met) offer(Q, got);
+        if (!whole && box_cost(Q) == 1.0) break;
     }
-    offer(Q, got);
     return best_q;
 }
 
@@ -228,13 +250,18 @@ std::vector<Cut> cut_items(const std::vector<ScanItem> &items, ScanLimits lim, u
     return out;
 }
 
-// The cut with fewer groups; program order where the search saves none (its groups are more even).
+// The cut with fewer groups (`lim.boxes`: of less time); program order where the search saves none (its groups are more even).
 std::vector<Cut> best_cut(const std::vector<ScanItem> &items, const ScanLimits &lim, uint64_t Q0, int n, bool windows,
                           bool search) {
     std::vector<Cut> plain = cut_items(items, lim, Q0, n, windows, false);
     if (!search || n <= lim.K || plain.size() < 3) return plain;
     std::vector<Cut> found = cut_items(items, lim, Q0, n, windows, true);
-    return found.size() < plain.size() ? found : plain;
+    auto time = [&](const std::vector<Cut> &cuts) {
+        double t = 0;
+        for (const Cut &c : cuts) t += lim.boxes ? box_cost(c.set) : 1.0;
+        return t;
+    };
+    return time(found) < time(plain) ? found : plain;
 }
 
 }  // namespace
@@ -267,6 +294,7 @@ Schedule build_schedule(int n, int K, int c, const std::vector<DevOp> &ops, bool
     lim.max_items = kMaxPassOps;
     lim.max_slots = kMaxPassSlots;
     lim.max_entries = limits.max_entries;
+    lim.boxes = limits.boxes;
     for (const ScanItem &it : items) lim.all |= it.touch;   // (a scan ends when they are blocked: idle qubits never are)
     for (const Cut &cut : best_cut(items, lim, (n <= K) ? all : ((uint64_t(1) << c) - 1), n, true, limits.search)) {
         const std::vector<int> &members = cut.members;
