@@ -387,6 +387,7 @@ struct RunTables {
     };
     std::vector<Gate> gates;
     std::vector<Entry> entries;
+    std::vector<int> wide;   // matrix table entries kept in FP64 (pipe::load_wide)
 
     static bool takes(const StageOp &so, int gid) {
         if (!on_expr(so).empty() || gid == GID_GP) return false;
@@ -414,11 +415,32 @@ struct RunTables {
         }
         return int(at);
     }
+    // The place among the FP64 entries of the M of a gate whose factors the threads make.
+    int add_wide(const StageOp &so) {
+        const int at = int(wide.size());
+        for (int e = 0; e < (so.kind == SK_DIAG2 ? 4 : 2); ++e) wide.push_back(so.moff + e);
+        return at;
+    }
+    // The run's gates with one factor for every thread (`same`: by place in the run), and the others.
+    static void split(const std::vector<const StageOp *> &run, const std::vector<int> &gids, std::vector<const StageOp *> &same,
+                      std::vector<size_t> &rest) {
+        for (size_t k = 0; k < run.size(); ++k) {
+            if (takes(*run[k], gids[k])) same.push_back(run[k]);
+            else rest.push_back(k);
+        }
+    }
+    // Shared memory: a table entry is 16 bytes in a forward pass and 8 in an adjoint, an FP64 entry 16; in table entries.
+    int units(bool adj) const {
+        return adj ? int((entries.size() + 1) / 2 * 2 + 2 * wide.size()) : int(entries.size() + wide.size());
+    }
     void declare(std::ostringstream &o) const {
-        if (entries.empty()) return;
-        o << "__device__ const pipe::RunGate run_gates[" << gates.size() << "] = {";
+        o << "constexpr int N_TAB = " << entries.size() << ", N_WIDE = " << wide.size() << ";\n";
+        o << "__device__ const unsigned short wide_src[" << std::max<size_t>(1, wide.size()) << "] = {";
+        for (int e : wide) o << e << ", ";
+        o << "};\n";
+        o << "__device__ const pipe::RunGate run_gates[" << std::max<size_t>(1, gates.size()) << "] = {";
         for (const Gate &g : gates) o << "{" << g.moff << ", " << g.p0 << ", " << g.p1 << ", " << g.ctrl << "}, ";
-        o << "};\n__device__ const pipe::RunEntry run_entries[" << entries.size() << "] = {";
+        o << "};\n__device__ const pipe::RunEntry run_entries[" << std::max<size_t>(1, entries.size()) << "] = {";
         for (const Entry &e : entries) o << "{" << e.first << ", " << e.n << ", " << e.idx << "}, ";
         o << "};\n";
     }
@@ -446,8 +468,10 @@ void emit_phase_run(std::ostringstream &o, const std::vector<const StageOp *> &r
     const bool adj = rows != nullptr;
     const int id = ctx.id++;
     const std::string u = "_" + std::to_string(id);
-    auto ent = [&](int M, const std::string &idx) {
-        const std::string e = "pipe::wide(mt[" + std::to_string(M) + " + " + idx + "])";
+    std::vector<int> wide(run.size(), -1);   // the gates' places among the pass's FP64 entries
+    auto ent = [&](size_t k, const std::string &idx) {
+        const std::string e = wide[k] >= 0 ? "wt[" + std::to_string(wide[k]) + " + " + idx + "]"
+                                           : "pipe::wide(mt[" + std::to_string(run[k]->moff) + " + " + idx + "])";
         return adj ? "cconj(" + e + ")" : e;
     };
     auto grads = [](const StageOp &so) { return so.n_angles ? so.grad_mask : 0; };
@@ -579,11 +603,8 @@ void emit_phase_run(std::ostringstream &o, const std::vector<const StageOp *> &r
         std::vector<const StageOp *> same;
         std::vector<size_t> rest;
         std::vector<int> bits;
-        for (size_t k = 0; k < run.size(); ++k) {
-            if (tables && RunTables::takes(*run[k], gids[k])) same.push_back(run[k]);
-            else rest.push_back(k);
-            own.push_back(k);
-        }
+        for (size_t k = 0; k < run.size(); ++k) own.push_back(k);
+        if (tables) RunTables::split(run, gids, same, rest);
         const int at = tables ? tables->add(same, bits) : -1;
         if (at >= 0) {
             own = rest;
@@ -602,6 +623,8 @@ void emit_phase_run(std::ostringstream &o, const std::vector<const StageOp *> &r
         }
     }
     if (own.empty()) return;
+    if (tables)
+        for (size_t k : own) wide[k] = tables->add_wide(*run[k]);
 
     // the thread's table over the register bits that the other gates depend on, and its scalar
     std::vector<int> tb;
@@ -640,15 +663,15 @@ void emit_phase_run(std::ostringstream &o, const std::vector<const StageOp *> &r
         auto sel = [&](const std::string &f) { return on.empty() ? f : "((" + on + ") ? " + f + " : cval<W>(1, 0))"; };
         const PhaseShape sh = phase_shape(so, gids[k]);
         if (sh == PH_OFF) {
-            const std::string f = sel(ent(so.moff, off_index(so, gids[k])));
+            const std::string f = sel(ent(k, off_index(so, gids[k])));
             o << "    sc = " << (ctx.sc ? "cmul(sc, " + f + ")" : f) << ";\n";
             ctx.sc = true;
         }
         if (sh != PH_BIT) continue;
         auto &p = pairs[phase_bit(so)];
         const auto ix = so.kind == SK_DIAG1 ? std::make_pair(std::string("0"), std::string("1")) : pair_index(so);
-        if (gids[k] != GID_PS) times(p.first, sel(ent(so.moff, ix.first)));   // (a phase shift's first entry is 1)
-        if (!mirrored) times(p.second, sel(ent(so.moff, ix.second)));
+        if (gids[k] != GID_PS) times(p.first, sel(ent(k, ix.first)));   // (a phase shift's first entry is 1)
+        if (!mirrored) times(p.second, sel(ent(k, ix.second)));
     }
     if (tb.empty()) return;
     // products over the bits' pairs, lowest bit first; of a mirrored table the half whose top bit is clear
@@ -672,7 +695,7 @@ void emit_phase_run(std::ostringstream &o, const std::vector<const StageOp *> &r
         const PhaseShape sh = phase_shape(so, gids[k]);
         if (sh == PH_PARITY) {
             for (int idx = 0; idx < nt; ++idx)
-                times(T[size_t(idx)], sel(ent(so.moff, (idx_bit(idx, so.dval[0]) ^ idx_bit(idx, so.dval[1])) ? "1" : "0")));
+                times(T[size_t(idx)], sel(ent(k, (idx_bit(idx, so.dval[0]) ^ idx_bit(idx, so.dval[1])) ? "1" : "0")));
         } else if (sh == PH_OTHER) {
             for (int idx = 0; idx < nt; ++idx) {
                 bool set = true;
@@ -685,7 +708,7 @@ void emit_phase_run(std::ostringstream &o, const std::vector<const StageOp *> &r
                                                             : "(" + off_bit_expr(so.dsrc[t], so.dval[t]) + ")";
                     r += t == 0 ? bit : " + 2 * " + bit;
                 }
-                times(T[size_t(idx)], sel(ent(so.moff, "(" + r + ")")));
+                times(T[size_t(idx)], sel(ent(k, "(" + r + ")")));
             }
         }
     }
@@ -1094,10 +1117,12 @@ void emit_ring_exit(std::ostringstream &o) {
 }
 
 // What a group makes of a new sample's matrix table: the pass norm and the runs' tables.
-void emit_load_derived(std::ostringstream &o, bool norm, int run_entries) {
+void emit_load_derived(std::ostringstream &o, bool norm, bool tables) {
     if (norm) o << "    pipe::pass_norm(ph, mt, a.mt, a.n_mt, tid);\n";
-    if (run_entries) o << "    pipe::load_runs(runs, mt, run_gates, run_entries, " << run_entries << ", tid, NT);\n";
-    if (norm || run_entries) o << "    pipe::consumers_sync(BAR, NT);\n";
+    if (tables)
+        o << "    if (N_TAB > 0) pipe::load_runs(runs, mt, run_gates, run_entries, N_TAB, tid, NT);\n"
+          << "    if (N_WIDE > 0) pipe::load_wide(wt, mt, wide_src, N_WIDE, tid, NT);\n";
+    if (norm || tables) o << "    pipe::consumers_sync(BAR, NT);\n";
 }
 
 std::string forward_source(const Schedule &s, const Pass &p, int precision, const std::vector<DevOp> &ops) {
@@ -1135,6 +1160,7 @@ std::string forward_source(const Schedule &s, const Pass &p, int precision, cons
     o << "  V *mt = reinterpret_cast<V *>(smem + NB * BUFB + grp * mtb);\n"
       << "  double *ph = reinterpret_cast<double *>(full + 16) + grp;\n"
       << "  pipe::Split *runs = reinterpret_cast<pipe::Split *>(full + 32) + grp * " << p.f_run_entries << ";\n"
+      << "  W *wt = reinterpret_cast<W *>(runs + N_TAB);   // matrix entries in FP64\n"
       << "  long long cached_b = -1;\n"
       << "  for (long long i = grp; i < cnt; i += G) {\n"
       << "   const long long w = first + i, b = w >> a.g.n_out;\n"
@@ -1144,7 +1170,7 @@ std::string forward_source(const Schedule &s, const Pass &p, int precision, cons
       << "   if (b != cached_b) {\n    pipe::consumers_sync(BAR, NT);\n"
       << "    pipe::load_mtab(mt, a.mt, a.n_mt, a.mats + b * a.mats_stride, a.cpool, tid, NT);\n"
       << "    cached_b = b;\n    pipe::consumers_sync(BAR, NT);\n";
-    emit_load_derived(o, norm, p.f_run_entries);
+    emit_load_derived(o, norm, p.f_run_entries > 0);
     o << "   }\n";
     emit_ring_wait(o);
     if (lp.relayout_in) {
@@ -1232,6 +1258,7 @@ std::string backward_source(const Schedule &s, const Pass &p, int precision, int
       << "  const unsigned scr = pipe::saddr(full + 32) + unsigned(grp * nw + warp) * " << scratch << "u;\n"
       << "  V *runs = reinterpret_cast<V *>(reinterpret_cast<unsigned char *>(full + 32) + G * nw * " << scratch << ") + grp * "
       << (shape.runs + 1) / 2 * 2 << ";\n"
+      << "  W *wt = reinterpret_cast<W *>(runs + (N_TAB + 1) / 2 * 2);   // matrix entries in FP64\n"
       << "  long long cached_b = -1;\n"
       << "  for (long long i = grp; i < cnt; i += G) {\n"
       << "   const long long w = first + i, b = w >> a.g.n_out;\n"
@@ -1241,7 +1268,7 @@ std::string backward_source(const Schedule &s, const Pass &p, int precision, int
       << "   if (b != cached_b) {\n    pipe::consumers_sync(BAR, NT);\n"
       << "    pipe::load_mtab(mt, a.mt, a.n_mt, a.mats + b * a.mats_stride, a.cpool, tid, NT);\n"
       << "    cached_b = b;\n    pipe::consumers_sync(BAR, NT);\n";
-    emit_load_derived(o, norm, shape.runs);
+    emit_load_derived(o, norm, shape.runs > 0);
     o << "   }\n";
     emit_ring_wait(o);
     if (lp.relayout_in) {
@@ -1463,13 +1490,15 @@ int jit_run_entries(const std::vector<const StageDesc *> &stages, const StageOp 
             *sd, sops, ops, adj,
             [&](const std::vector<const StageOp *> &run, const std::vector<int> &gids) {
                 std::vector<const StageOp *> same;
+                std::vector<size_t> rest;
                 std::vector<int> bits;
+                RunTables::split(run, gids, same, rest);
+                const bool table = tables.add(same, bits) >= 0;
                 for (size_t k = 0; k < run.size(); ++k)
-                    if (RunTables::takes(*run[k], gids[k])) same.push_back(run[k]);
-                tables.add(same, bits);
+                    if (!table || std::find(rest.begin(), rest.end(), k) != rest.end()) tables.add_wide(*run[k]);
             },
             [](const StageOp &) {});
-    return int(tables.entries.size());
+    return tables.units(adj);
 }
 
 std::string jit_forward_source(const Schedule &s, const Pass &p, int precision, const std::vector<DevOp> &ops) {
