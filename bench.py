@@ -126,7 +126,7 @@ def _peaks():
 
 # DRAM bytes per state byte moved by one adjoint pass launch (psi read, lambda read + write: 3 x
 # S*B algorithmic), from an ncu capture of the same kernel on the HEA 24-qubit, batch-2 case; a
-# launch's traffic grows in proportion to the state bytes it processes (760.9 and 761.6 MB read +
+# launch's traffic grows in proportion to the state bytes it processes (763.4 and 763.0 MB read +
 # written for S*B = 268.4 MB in the two captured launches).  None: not captured for
 # the kernels built from the current sources.
 ADJ_DRAM_BYTES_PER_STATE_BYTE = 2.84

@@ -923,8 +923,8 @@ void emit_relayout(std::ostringstream &o, const PassPlan &pl, int K, int TB, int
 // warps keeps 128 registers per thread.  Defaults, measured on gradients of the 26-qubit, 12-layer ansatz (batch 2),
 // the 20-qubit classifier (64 samples) and QAOA on 26 vertices: the adjoint takes two groups and three buffers; the
 // complex64 forward pass, with 16 amplitudes per thread, one group and two buffers, so that three blocks share
-// an SM (13.4, 5.4 and 7.8 ms; two groups and three buffers 14.2, 5.2 and 8.3; one group and three buffers
-// 15.1, 5.4 and 8.0); complex128, whose tiles leave room for one block, two groups and three buffers.
+// an SM (whole gradients 53.9, 37.2 and 26.3 ms; two groups and three buffers 53.6, 37.4 and 26.4; one group and three buffers
+// 54.0, 37.5 and 26.3); complex128, whose tiles leave room for one block, two groups and three buffers.
 // MQB_PIPE_{FWD,BWD}_{GROUPS,BUFFERS} override them (tuning).
 int env_int(const char *name, int dflt, int lo, int hi) {
     const char *e = std::getenv(name);

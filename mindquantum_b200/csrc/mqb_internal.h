@@ -232,9 +232,8 @@ int default_tile_bits(int precision, int n_states_in_tile);
 // Register bits of the fused kernels: forward passes, and backward passes with n_hams lambdas.
 int fwd_reg_bits(int precision);
 // The same for the generated forward kernels: 4 for complex64.  16 amplitudes per thread take half the code of 32,
-// which is straight-line and bound by instruction fetch as much as by arithmetic, at the price of more
-// stages: 26 qubits x 12 layers 14.1 -> 13.2 ms of forward passes (batch 2), the 20-qubit classifier 6.6 -> 5.4, QAOA
-// on 26 vertices 9.3 -> 7.8; compiling takes half the time.
+// which is straight-line, at the price of more stages: whole gradients of 26 qubits x 12 layers (batch 2) 53.9 against 54.8 ms
+// with 32, the 20-qubit classifier 37.2 against 37.6, QAOA on 26 vertices 26.3 against 27.0; compiling takes half the time.
 int jit_fwd_reg_bits(int precision);
 int bwd_reg_bits(int precision, int n_hams);
 
